@@ -104,6 +104,9 @@ bool make_opts(const gamera_no_advance_options *o, bool have_background,
   O.hogs_h = s.hydro_hogs_coefficient;
   O.hogs_m = s.magnetic_hogs_coefficient;
   O.s_c = s.light_speed;
+  O.s_igm1 = 1.0 / (s.gamma - 1.0);
+  O.s_igm1_f32 = 1.0f / ((float)s.gamma - 1.0f);
+  O.s_ic2 = s.use_boris ? 1.0 / (s.light_speed * s.light_speed) : 0.0;
   O.s_mhd = s.use_mhd;
   O.hogs = s.use_hogs;
   O.s_boris = s.use_boris;
@@ -290,21 +293,14 @@ int run_step(gcs_context *ctx, const gcs::Opts &O, int driver_mode,
     gcs::launch_edge_sync(X, s);
     mk.mark(kSlotEdgeSync);
   }
-  gcs::launch_update(X, O, s);
+  gcs::launch_update(X, O, driver_mode && !post_control, s);
   mk.mark(kSlotUpdate);
-  if (O.u_mhd) {
-    gcs::launch_seam_sync(X, 1, s);
-    mk.mark(kSlotSeamPhiFinal);
-    gcs::launch_recover(X, O, driver_mode && !post_control, s);
-    mk.mark(kSlotRecover);
-  }
   if (post_control) {
     // the Earth drivers' post-step pressure control with this step's dt,
     // fused with the CFL reduction of the controlled state
     gcs::launch_pressure_control(C, C.pc, 0.0, &O, s);
   }
   if (driver_mode) {
-    gcs::launch_count_step(X, s);
     gcs::launch_next_dt(X, O.dt_fraction, s);
     mk.mark(kSlotDt);
   }

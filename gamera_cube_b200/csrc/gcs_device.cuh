@@ -141,6 +141,8 @@ struct StepParams {
 // (nonorthogonal_step.h:57-65) and CFL time step (:67-76).
 struct Opts {
   double s_gamma, s_rho_floor, s_p_floor, pdm, hogs_h, hogs_m, s_c;
+  double s_igm1, s_ic2;          // 1 / (gamma - 1); 1 / c^2 with Boris, else 0
+  float s_igm1_f32;              // 1 / (gamma - 1) of the FP32 gamma, in FP32
   bool s_mhd, hogs, s_boris, s_bg;
   double e_rho_floor, e_pdm, e_diff, e_c, e_cfl;
   bool e_boris, e_bg;

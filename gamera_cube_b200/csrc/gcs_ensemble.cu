@@ -340,6 +340,10 @@ gcs_ensemble *gcs_ensemble_create(const gcs_ensemble_config *cfg) {
       E->prev[i] = p;
     }
     E->runs[i] = ctx;
+    // one graph node per face or edge family: the branches of the step graph
+    // fill the GPU between them, and the node count of the graph stays what
+    // gcs_ensemble_graph_info has reported
+    ctx->c.X.split_families = 1;
     if (rc != 0) {
       char msg[300];
       snprintf(msg, sizeof(msg), "run %d: %s", i, ctx->c.error);

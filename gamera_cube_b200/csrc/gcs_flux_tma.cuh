@@ -1,5 +1,5 @@
 // Face-flux sweep with the eight-cell Up7 stencil staged in shared memory by
-// TMA (nonorthogonal_sweep.c:408-548, the arithmetic of k_flux).
+// TMA (nonorthogonal_sweep.c:408-548, the arithmetic of k_flux: face_flux).
 //
 // A thread block is persistent: it walks a list of tiles, each tile a
 // FX x FY patch of faces of one direction d (FX consecutive faces along the
@@ -27,6 +27,7 @@
 #include <cuda.h>
 
 #include "gcs_kernel_util.cuh"
+#include "gcs_face_flux.cuh"
 #include "gcs_kernels.cuh"
 #include "gcs_physics.cuh"
 
@@ -163,126 +164,22 @@ __device__ __forceinline__ void issue_tile(const FluxMaps &maps, const Dims &D,
   }
 }
 
-// The flux of one face from the staged stencil (same operations as k_flux).
+// Stencil cells of a face in a stage buffer.
 template <int d, typename T>
-__device__ __forceinline__ void staged_face(const T *sm, int s0, const Dims &D,
-                                            const DevState &S, const Bulk<T> &B,
-                                            const Opts &O, DevStatus *st, int f, int i,
-                                            int j, int k) {
-  using Sh = FluxTile<d, T>;
-  const long long c = f * D.Nn + D.node(i, j, k);
-  const long long cb = B.at(f, D.node(i, j, k));   // index of the Bulk arrays
-  const long long sd = D.stride(d);
-  const T iv = B.iv[d][cb];
-  if (isnan(iv)) {
-    fail(st, kStageReconstruct, d, f, i, j, k);
-    return;
+struct StagedStencil {
+  const T *p;
+  __device__ __forceinline__ void load(int v, T q[8]) const {
+    using Sh = FluxTile<d, T>;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) q[n] = p[v * Sh::CELLS + n * Sh::STEP];
   }
-  const T riv = T(1.0) / iv;
-  const T pdm = (T)O.pdm;
-  const T *svol = sm + 8 * Sh::CELLS + s0;
-  T vol[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) vol[n] = svol[n * Sh::STEP];
-  PrimT<T> st2[2];
-  {
-    T q[8], l, r;
-    bool ok = true;
-    const T *sp = sm + s0;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      q[n] = sp[n * Sh::STEP];
-      ok = ok && !isnan(q[n]);
-    }
-    if (!ok) {
-      fail(st, kStageReconstruct, d, f, i, j, k);
-      return;
-    }
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].rho = l; st2[1].rho = r;
-    sp += Sh::CELLS;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = sp[n * Sh::STEP];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vx = l; st2[1].vx = r;
-    sp += Sh::CELLS;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = sp[n * Sh::STEP];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vy = l; st2[1].vy = r;
-    sp += Sh::CELLS;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = sp[n * Sh::STEP];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vz = l; st2[1].vz = r;
-    sp += Sh::CELLS;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = sp[n * Sh::STEP];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].p = l; st2[1].p = r;
-  }
-  T mag[2][3] = {{T(0.0), T(0.0), T(0.0)}, {T(0.0), T(0.0), T(0.0)}};
-  if (O.s_mhd) {
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      const T *sp = sm + (5 + m) * Sh::CELLS + s0;
-      T q[8];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) q[n] = sp[n * Sh::STEP];
-      up7_pdm_rcp(vol, q, riv, pdm, &mag[0][m], &mag[1][m]);
-    }
-  }
-  FaceFrame<T> fr;
-  fr.nx = B.fn[d][0][cb]; fr.ny = B.fn[d][1][cb]; fr.nz = B.fn[d][2][cb];
-  fr.t1x = B.ft1[d][0][cb]; fr.t1y = B.ft1[d][1][cb]; fr.t1z = B.ft1[d][2][cb];
-  fr.t2x = B.ft2[d][0][cb]; fr.t2y = B.ft2[d][1][cb]; fr.t2z = B.ft2[d][2][cb];
-  FluidFlux<T> fl;
-  if (kinetic_fluid_flux(st2, (T)O.s_gamma, fr, &fl)) {
-    fail(st, kStageKineticFluid, d, f, i, j, k);
-    return;
-  }
-  MaxwellFlux<T> mx;
-  mx.m[0] = mx.m[1] = mx.m[2] = T(0.0);
-  if (O.s_mhd) {
-    const T bn = B.BN[d][cb];
-    T b0[3] = {T(0.0), T(0.0), T(0.0)};
-    T b0n = T(0.0);
-    if (O.s_bg) {
-      b0[0] = B.fb0[d][0][cb];
-      b0[1] = B.fb0[d][1][cb];
-      b0[2] = B.fb0[d][2][cb];
-      b0n = B.fb0n[d][cb];
-    }
-    if (kinetic_maxwell_flux(st2, mag, bn, fr, O.s_bg, b0, b0n, O.s_boris, (T)O.s_c,
-                             fl.vn, &mx)) {
-      fail(st, kStageKineticMaxwell, d, f, i, j, k);
-      return;
-    }
-    if (O.hogs)
-      apply_hogs(&fl, &mx, (T)O.hogs_h, (T)O.hogs_m, O.s_boris, (T)O.s_c);
-    if (O.hogs && O.s_boris) {
-      bool applied;
-      T speed;
-      if (emergency_diffusion(&fl, st2, S.Up, c - sd, c, (T)O.s_c, &applied, &speed)) {
-        fail(st, kStageEmergency, d, f, i, j, k);
-        return;
-      }
-      if (applied) {
-        atomicAdd(&st->emergency_count[f], 1ULL);
-        atomicMax(&st->emergency_max_bits[f],
-                  (unsigned long long)__double_as_longlong((double)speed));
-      }
-    }
-  }
-  const T area = B.area[d][cb];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) B.F[d][m][c] = (double)(area * fl.f[m]);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) B.M[d][m][c] = (double)(area * mx.m[m]);
-}
+  __device__ __forceinline__ void volume(T q[8]) const { load(8, q); }
+  __device__ __forceinline__ void prim(int m, T q[8]) const { load(m, q); }
+  __device__ __forceinline__ void field(int m, T q[8]) const { load(5 + m, q); }
+};
 
 // Face (x, y) of tile c: x along k, y along the second tile axis.
-template <int d, typename T>
+template <int d, bool kOrtho, typename T>
 __device__ __forceinline__ void tile_face(const T *sm, const TileCoord &c, int x, int y,
                                           const FluxTiles &L, const Dims &D,
                                           const DevState &S, const Bulk<T> &B,
@@ -305,7 +202,9 @@ __device__ __forceinline__ void tile_face(const T *sm, const TileCoord &c, int x
     k = D.g + c.b + x;
     s0 = y * Sh::BX + x;
   }
-  staged_face<d, T>(sm, s0, D, S, B, O, st, c.f, i, j, k);
+  const FaceAt at{c.f, i, j, k, (unsigned)(c.f * D.Nn + D.node(i, j, k)),
+                  (unsigned)B.at(c.f, D.node(i, j, k))};
+  face_flux<kOrtho, T>(d, StagedStencil<d, T>{sm + s0}, D, S, B, O, st, at);
 }
 
 // Warps of a staged flux block.  They share the stage buffers but never wait
@@ -313,7 +212,7 @@ __device__ __forceinline__ void tile_face(const T *sm, const TileCoord &c, int x
 // to read, and the last warp to finish reading a stage issues its refill
 // (the tile kStages iterations ahead).  The extra faces of a last tile along
 // the sweep axis go to one warp, a different warp on each iteration.
-template <int d, typename T>
+template <int d, bool kOrtho, typename T>
 __global__ void __launch_bounds__(256, FluxTile<d, T>::MIN_BLOCKS)
     k_flux_tma(const __grid_constant__ FluxMaps maps, Dims D, DevState S, Bulk<T> B,
                Opts O, DevStatus *st, FluxTiles L) {
@@ -388,7 +287,7 @@ __global__ void __launch_bounds__(256, FluxTile<d, T>::MIN_BLOCKS)
         y = Sh::FY;
         on = c.fa > Sh::FY && lane < c.fb;
       }
-      if (on) tile_face<d, T>(sm, c, x, y, L, D, S, B, O, st);
+      if (on) tile_face<d, kOrtho, T>(sm, c, x, y, L, D, S, B, O, st);
     }
     // this warp is done with the stage; the last warp refills it
     __syncwarp();
@@ -455,18 +354,18 @@ FluxTiles flux_tiles(const Dims &D, int i0, int i1) {
 // Persistent grid of the staged flux sweep: resident blocks per SM times
 // SMs, found once per process (outside any stream capture: the first call
 // comes from prepare_flux_tma at context set-up).
-template <int d, typename T>
+template <int d, bool kOrtho, typename T>
 int flux_tma_blocks() {
   using Sh = FluxTile<d, T>;
   static int blocks = 0;
   if (blocks == 0) {
-    if (cudaFuncSetAttribute(k_flux_tma<d, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(k_flux_tma<d, kOrtho, T>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)Sh::SMEM) != cudaSuccess)
       return -1;
     int per_sm = 0, sms = 0, dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flux_tma<d, T>,
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_flux_tma<d, kOrtho, T>,
                                                       Sh::THREADS, Sh::SMEM) != cudaSuccess ||
         per_sm <= 0 || sms <= 0)
       return -1;
@@ -477,8 +376,9 @@ int flux_tma_blocks() {
 
 template <typename T>
 int prepare_flux_tma() {
-  return (flux_tma_blocks<0, T>() > 0 && flux_tma_blocks<1, T>() > 0 &&
-          flux_tma_blocks<2, T>() > 0) ? 0 : -1;
+  return (flux_tma_blocks<0, true, T>() > 0 && flux_tma_blocks<1, true, T>() > 0 &&
+          flux_tma_blocks<2, true, T>() > 0 && flux_tma_blocks<0, false, T>() > 0 &&
+          flux_tma_blocks<1, false, T>() > 0 && flux_tma_blocks<2, false, T>() > 0) ? 0 : -1;
 }
 
 // Launch of the staged flux sweep of direction d over [i0, i1).
@@ -499,14 +399,15 @@ void launch_flux_tma(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int 
       launch_set_failure(X, kStageTileCopy, d, s);
       return;
     }
-  const int blocks = flux_tma_blocks<d, T>();
+  const bool ortho = X.ortho && sizeof(T) == 8;  // as the per-face sweep
+  const int blocks = ortho ? flux_tma_blocks<d, true, T>() : flux_tma_blocks<d, false, T>();
   if (blocks <= 0) {
     launch_set_failure(X, kStageTileCopy, d, s);
     return;
   }
   const long long grid = L.count < blocks ? L.count : blocks;
-  k_flux_tma<d, T><<<(unsigned)grid, Sh::THREADS, Sh::SMEM, s>>>(maps, D, X.S, B, O,
-                                                                  X.status, L);
+  (ortho ? k_flux_tma<d, true, T> : k_flux_tma<d, false, T>)
+      <<<(unsigned)grid, Sh::THREADS, Sh::SMEM, s>>>(maps, D, X.S, B, O, X.status, L);
 }
 
 }  // namespace gcs

@@ -213,133 +213,6 @@ __global__ void k_halo_faces(Dims D, const HaloFace *plan, long long count,
 }
 
 // ---------------------------------------------------------------------------
-// Predictor over every cell and face incl. ghosts
-// (nonorthogonal_step.c:379-419): U~ = prim^-1(P + r (P - P_old)),
-// Phi~ = Phi + r (Phi - Phi_old), B~ = recover(Phi~); plus the per-cell
-// momentum weights (V m)/max(rho, floor) of the EMF face velocities
-// (nonorthogonal_sweep.c:223-249), which depend on U~ only.  Also stores,
-// once per cell and face, two quantities every sweep stencil reads many
-// times: the primitive state of U~ under the sweep options
-// (nonorthogonal_sweep.c:144-149, rho = NaN marks a failed conversion) and
-// the face-normal field Phi~ / area (nonorthogonal_sweep.c:466-467, 391).
-// Final B recovery on every cell (cubedsphere_step.c:142-152), optionally
-// fused with the CFL time-step reduction of the next step
-// (nonorthogonal_step.c:449-525) over active cells.  mode bit 0: recover
-// and store B; bit 1: CFL reduction (with the stored B when bit 0 is clear).
-__global__ void __launch_bounds__(256, 4) k_recover(Dims D, DevState S, DevGeom G,
-                                                 DevBg BG, Opts O, int mode,
-                                                 DevStatus *st) {
-  // No early return: every thread reaches the block reduction below.
-  const bool skip = failed(st);
-  const int with_cfl = mode & 2;
-  int f, i, j, k;
-  const Box b{0, 0, 0, D.E1, D.E2, D.E0};
-  double cand = DBL_MAX;
-  if (!skip && box_coord(b, &f, &i, &j, &k)) {
-    const long long c = f * D.Nn + D.node(i, j, k);
-    double bn[3];
-    bool ok = true;
-    if (mode & 1) {
-      double phi[6];
-      const long long sdir[3] = {D.stride(0), D.stride(1), 1};
-#pragma unroll
-      for (int d = 0; d < 3; ++d) {
-        phi[2 * d] = S.P[d][c];
-        phi[2 * d + 1] = S.P[d][c + sdir[d]];
-      }
-      ok = recover_cell(G, c, phi, bn);
-      if (!ok) {
-        fail(st, kStageRecoverFinal, 0, f, i, j, k);
-      } else {
-#pragma unroll
-        for (int m = 0; m < 3; ++m) S.B[m][c] = bn[m];
-      }
-    } else {
-#pragma unroll
-      for (int m = 0; m < 3; ++m) bn[m] = S.B[m][c];
-    }
-    if (ok) {
-      if (with_cfl && i >= D.g && i < D.g + D.nr && j >= D.g &&
-          j < D.g + D.n && k >= D.g && k < D.g + D.n) {
-        double u[5];
-#pragma unroll
-        for (int m = 0; m < 5; ++m) u[m] = S.U[m][c];
-        Prim p;
-        if (cons_to_prim(u, O.t_gamma, O.t_rho_floor, O.t_p_floor, &p)) {
-          fail(st, kStageTimestep, 0, f, i, j, k);
-        } else {
-          const double cs = sqrt(O.t_gamma * p.p / p.rho);
-          double va = 0.0;
-          if (O.t_mhd) {
-            double bx = bn[0], by = bn[1], bz = bn[2];
-            if (O.t_bg) {
-              bx = bn[0] + BG.b0[0][c];
-              by = bn[1] + BG.b0[1][c];
-              bz = bn[2] + BG.b0[2][c];
-            }
-            double s2 = 0.0;
-            s2 += bx * bx;
-            s2 += by * by;
-            s2 += bz * bz;
-            va = sqrt(s2) / sqrt(p.rho);
-            if (O.t_boris) va = O.t_c * va / hypot(O.t_c, va);
-          }
-          double v2 = 0.0;
-          v2 += p.vx * p.vx;
-          v2 += p.vy * p.vy;
-          v2 += p.vz * p.vz;
-          const double speed = sqrt(v2) + hypot(cs, va);
-          const double cand0 = O.t_cfl * G.cflmin[c] / speed;
-          if (!isfinite(cand0) || cand0 <= 0.0)
-            fail(st, kStageTimestep, 0, f, i, j, k);
-          else
-            cand = cand0;
-        }
-      }
-    }
-  }
-  if (!with_cfl) return;
-  // block min (positive doubles order as unsigned 64-bit integers)
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1)
-    cand = fmin(cand, __shfl_down_sync(0xffffffffu, cand, o));
-  __shared__ double wmin[8];
-  const int lt = threadIdx.y * blockDim.x + threadIdx.x;
-  const int lane = lt & 31, warp = lt >> 5;
-  if (lane == 0) wmin[warp] = cand;
-  __syncthreads();
-  if (warp == 0) {
-    cand = lane < (int)((blockDim.x * blockDim.y) >> 5) ? wmin[lane] : DBL_MAX;
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1)
-      cand = fmin(cand, __shfl_down_sync(0xffffffffu, cand, o));
-    if (lane == 0 && cand < DBL_MAX)
-      atomicMin(&st->cfl_min_bits,
-                (unsigned long long)__double_as_longlong(cand));
-  }
-}
-
-// Driver-mode time step (test_cubedsphere_dipole_background.c:593-670):
-// dt = min(fraction * cfl_min, 1.25 dt_prev), ratio = 0.5 dt / dt_prev
-// (0 on the first step).  Resets the reduction for the next step.
-__global__ void k_next_dt(StepParams *prm, DevStatus *st, double fraction) {
-  const double local = __longlong_as_double((long long)st->cfl_min_bits);
-  prm->cfl_min = local;
-  const double prev = prm->dt;
-  double dt = fraction * local;
-  if (prm->step > 0) dt = fmin(dt, 1.25 * prev);
-  prm->ratio = prm->step > 0 ? 0.5 * dt / prev : 0.0;
-  prm->dt_prev = prev;
-  prm->dt = dt;
-  st->cfl_min_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
-}
-
-__global__ void k_count_step(StepParams *prm) {
-  prm->time += prm->dt;
-  prm->step += 1;
-}
-
-// ---------------------------------------------------------------------------
 // Host-side launchers.
 
 Bulk<double> bulk64(const Ctx &X) {
@@ -463,32 +336,22 @@ void launch_edge_sync(const Ctx &X, cudaStream_t s) {
         X.D, X.edge_offsets, X.edge_members, X.n_edge_groups, X.S, X.status);
 }
 
-void launch_update(const Ctx &X, const Opts &O, cudaStream_t s) {
+void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s) {
   const Dims &D = X.D;
   const Tile t = X.tile[kTileCt], tu = X.tile[kTileUpdate];
-  k_ct<0><<<tile_grid(D.E0 + 1, D.E1, D.E2, t), tile_block(t), 0, s>>>(
-      D, X.S, O, X.params, X.status);
-  k_ct<1><<<tile_grid(D.E0, D.E1 + 1, D.E2, t), tile_block(t), 0, s>>>(
-      D, X.S, O, X.params, X.status);
-  k_ct<2><<<tile_grid(D.E0, D.E1, D.E2 + 1, t), tile_block(t), 0, s>>>(
-      D, X.S, O, X.params, X.status);
+  for (int d = X.split_families ? 0 : -1; d < (X.split_families ? 3 : 0); ++d)
+    k_ct<<<tile_grid(D.E0 + 1, D.E1 + 1, D.E2 + 1, t), tile_block(t), 0, s>>>(
+        D, X.S, O, d < 0 ? 7 : 1 << d, X.params, X.status);
+  if (O.u_mhd) launch_seam_sync(X, 1, s);
   k_update<<<tile_grid(D.E0, D.E1, D.E2, tu), tile_block(tu), 0, s>>>(
-      D, X.S, X.G, X.BG, O, X.params, X.status);
-}
-
-void launch_recover(const Ctx &X, const Opts &O, int with_cfl,
-                    cudaStream_t s) {
-  const Dims &D = X.D;
-  const Tile t = X.tile[kTileRecover];
-  k_recover<<<tile_grid(D.E0, D.E1, D.E2, t), tile_block(t), 0, s>>>(
-      D, X.S, X.G, X.BG, O, 1 | (with_cfl ? 2 : 0), X.status);
+      D, X.S, X.G, X.BG, O, with_cfl && O.u_mhd, X.params, X.status);
 }
 
 void launch_timestep(const Ctx &X, const Opts &O, cudaStream_t s) {
   const Dims &D = X.D;
   const Tile t = X.tile[kTileRecover];
-  k_recover<<<tile_grid(D.E0, D.E1, D.E2, t), tile_block(t), 0, s>>>(
-      D, X.S, X.G, X.BG, O, 2, X.status);
+  k_timestep<<<tile_grid(D.nr, D.n, D.n, t), tile_block(t), 0, s>>>(D, X.S, X.G, X.BG, O,
+                                                                  X.status);
 }
 
 __global__ void k_set_failure(DevStatus *st, int stage, int dir) {
@@ -503,10 +366,6 @@ void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s) {
   k_next_dt<<<1, 1, 0, s>>>(X.params, X.status, fraction);
 }
 
-void launch_count_step(const Ctx &X, cudaStream_t s) {
-  k_count_step<<<1, 1, 0, s>>>(X.params);
-}
-
 // Whole step in reference order.
 void launch_step(const Ctx &X, const Opts &O, int driver_mode,
                  cudaStream_t s) {
@@ -519,13 +378,8 @@ void launch_step(const Ctx &X, const Opts &O, int driver_mode,
     launch_emf(X, O, s);
     launch_edge_sync(X, s);
   }
-  launch_update(X, O, s);
-  if (O.u_mhd) launch_seam_sync(X, 1, s);
-  if (O.u_mhd) launch_recover(X, O, driver_mode, s);
-  if (driver_mode) {
-    launch_count_step(X, s);
-    launch_next_dt(X, O.dt_fraction, s);
-  }
+  launch_update(X, O, driver_mode, s);
+  if (driver_mode) launch_next_dt(X, O.dt_fraction, s);
 }
 
 }  // namespace gcs

@@ -39,6 +39,8 @@ struct Ctx {
   int n_edge_groups = 0;
   StepParams *params = nullptr;   // device
   DevStatus *status = nullptr;    // device
+  int ortho = 0;                  // 1: every active face frame is orthonormal
+  int split_families = 0;         // 1: a launch per face or edge family (ensembles)
   int flux_staged = 0;            // 1: TMA-staged flux sweeps (gcs_flux_tma.cuh)
   int bulk = 0;                   // 1: FP32-bulk sweeps (B32)
   int bulk_split = 0;             // radial layers [0, bulk_split) stay FP64
@@ -84,11 +86,10 @@ void launch_emf(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_face_velocities(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_edge_emfs(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_edge_sync(const Ctx &X, cudaStream_t s);
-void launch_update(const Ctx &X, const Opts &O, cudaStream_t s);
-void launch_recover(const Ctx &X, const Opts &O, int with_cfl,
-                    cudaStream_t s);
+// CT, the seam sync of Phi, then the cell update with the final recovery;
+// with_cfl: also the CFL reduction of the new state into status.
+void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s);
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s);
-void launch_count_step(const Ctx &X, cudaStream_t s);
 void launch_step(const Ctx &X, const Opts &O, int driver_mode,
                  cudaStream_t s);
 // CFL reduction alone (nonorthogonal_step.c:449-525) into status.

@@ -175,6 +175,29 @@ __global__ void k_derive_iv(Dims D, int d, DevGeom G) {
   G.iv[d][c] = (isfinite(iv) && fabs(iv) > DBL_MIN) ? iv : NAN;
 }
 
+// Set *general where the frame of an active face is not orthonormal to
+// rounding (1e-13, some hundred times the rounding of a normalised frame):
+// the flux sweeps then keep the form that reads the tangents.  The
+// reference's geometry makes orthonormal frames; a caller's grid need not.
+__global__ void k_check_frames(Dims D, int d, DevGeom G, int *general) {
+  int i, j, k;
+  if (box_index(&i, &j, &k, D.n + (d == 1), D.n + (d == 2), D.nr + (d == 0)) < 0) return;
+  const long long c = blockIdx.y * D.Nn + D.node(i + D.g, j + D.g, k + D.g);
+  double v[3][3];
+  for (int q = 0; q < 3; ++q) {
+    v[0][q] = G.fn[d][q][c];
+    v[1][q] = G.ft1[d][q][c];
+    v[2][q] = G.ft2[d][q][c];
+  }
+  bool ok = true;
+  for (int a = 0; a < 3; ++a)
+    for (int b = a; b < 3; ++b) {
+      const double p = dot3(v[a][0], v[a][1], v[a][2], v[b][0], v[b][1], v[b][2]);
+      ok = ok && fabs(p - (a == b ? 1.0 : 0.0)) <= 1e-13;
+    }
+  if (!ok) *general = 1;
+}
+
 // nonorthogonal_operators.c:81-113: area-weighted central6 face normal at the
 // edge, projected on the edge tangents and normalised.
 __device__ bool transverse_normal(const DevGeom &G, int fam, long long c,
@@ -560,8 +583,17 @@ int Context::derive() {
     k_derive_edges<<<dim3(blocks_for(ec, 128), kFaces), 128, 0, stream>>>(
         D, e, G);
   }
+  int general = 0;
+  GCS_TRY(cudaMemsetAsync(staging, 0, sizeof(int), stream));
+  for (int d = 0; d < 3; ++d) {
+    const long long fc = (long long)(D.nr + (d == 0)) * (D.n + (d == 1)) * (D.n + (d == 2));
+    k_check_frames<<<dim3(blocks_for(fc, 128), kFaces), 128, 0, stream>>>(D, d, G,
+                                                                          (int *)staging);
+  }
   GCS_TRY(cudaGetLastError());
+  GCS_TRY(cudaMemcpyAsync(&general, staging, sizeof(int), cudaMemcpyDeviceToHost, stream));
   GCS_TRY(cudaStreamSynchronize(stream));
+  X.ortho = general ? 0 : 1;
   return 0;
 }
 

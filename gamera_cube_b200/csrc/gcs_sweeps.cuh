@@ -16,16 +16,29 @@
 #pragma once
 
 #ifndef GCS_F32_FLUX_BLOCKS
-#define GCS_F32_FLUX_BLOCKS 8
+#define GCS_F32_FLUX_BLOCKS 6
 #endif
 #ifndef GCS_F32_EDGE_BLOCKS
 #define GCS_F32_EDGE_BLOCKS 8
+#endif
+#ifndef GCS_PREDICT_BLOCKS
+#define GCS_PREDICT_BLOCKS 4
+#endif
+#ifndef GCS_UPDATE_BLOCKS
+#define GCS_UPDATE_BLOCKS 4
+#endif
+#ifndef GCS_FLUX_BLOCKS
+#define GCS_FLUX_BLOCKS 4
+#endif
+#ifndef GCS_EDGE_BLOCKS
+#define GCS_EDGE_BLOCKS 6
 #endif
 
 
 #include "gcs_kernel_util.cuh"
 #include "gcs_kernels.cuh"
 #include "gcs_physics.cuh"
+#include "gcs_face_flux.cuh"
 #include "gcs_flux_tma.cuh"
 
 namespace gcs {
@@ -37,77 +50,89 @@ namespace gcs {
 // B~ in FP64; primitives of U~ with the sweep options (rho NaN where the
 // conversion fails), Phi~/area and the EMF weights V m / max(rho, floor)
 // for the sweeps, in FP64 and (bulk) FP32.
-__global__ void k_predict(Dims D, DevState S, DevGeom G, Bulk<float> B32, int bulk,
+__global__ void __launch_bounds__(256, GCS_PREDICT_BLOCKS) k_predict(Dims D, DevState S, DevGeom G, Bulk<float> B32, int bulk,
                           Opts O, const StepParams *prm, DevStatus *st) {
-  if (failed(st)) return;
+  const unsigned long long first = failure_word(st);
   int f, i, j, k;
   const Box b{0, 0, 0, D.N1, D.N2, D.E0 + 1};
   if (!box_coord(b, &f, &i, &j, &k)) return;
   const double r = prm->ratio;
-  const long long c = f * D.Nn + D.node(i, j, k);
+  const unsigned c = (unsigned)(f * D.Nn + D.node(i, j, k));
   // FP32 copies exist for the layers [B32.lo, N0) only
   const bool wb = bulk && i >= B32.lo;
-  const long long cb = wb ? B32.at(f, D.node(i, j, k)) : 0;
+  const unsigned cb = wb ? (unsigned)B32.at(f, D.node(i, j, k)) : 0;
   const bool cell = i < D.E0 && j < D.E1 && k < D.E2;
   const int coord[3] = {i, j, k};
+  double phi[6], bn[3];
+  bool in[3];
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
-    bool in = true;
+    in[d] = true;
 #pragma unroll
-    for (int a = 0; a < 3; ++a) in = in && coord[a] < D.ext(a) + (a == d ? 1 : 0);
-    if (in) {
-      const double pp = S.P[d][c] + r * (S.P[d][c] - S.Po[d][c]);
-      S.Pp[d][c] = pp;
-      const double bn = pp / G.area[d][c];
-      S.BN[d][c] = bn;
-      if (wb) B32.BN[d][cb] = (float)bn;
+    for (int a = 0; a < 3; ++a) in[d] = in[d] && coord[a] < D.ext(a) + (a == d ? 1 : 0);
+    phi[2 * d] = bn[d] = 0.0;
+    if (in[d]) {
+      const double p = S.P[d][c];
+      phi[2 * d] = p + r * (p - S.Po[d][c]);
+      bn[d] = phi[2 * d] / G.area[d][c];
     }
   }
-  if (!cell) return;
-  double uo[5], uc[5], up[5];
+  double up[5], bp[3], prv[5], v = 0.0;
+  bool ok = true, recovered = true;
+  if (cell) {
+    double uo[5], uc[5];
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    uo[m] = S.Uo[m][c];
-    uc[m] = S.U[m][c];
+    for (int m = 0; m < 5; ++m) {
+      uo[m] = S.Uo[m][c];
+      uc[m] = S.U[m][c];
+    }
+#pragma unroll
+    for (int d = 0; d < 3; ++d) {
+      const unsigned u = c + (unsigned)D.stride(d);
+      const double p = S.P[d][u];
+      phi[2 * d + 1] = p + r * (p - S.Po[d][u]);
+    }
+    v = G.vol[c];
+    recovered = recover_cell(G, c, phi, bp);
+    ok = predict_cell(uo, uc, r, O.u_gamma, O.u_rho_floor, O.u_p_floor, up) == 0;
+    Prim pr;
+    if (cons_to_prim(up, O.s_gamma, O.s_rho_floor, O.s_p_floor, &pr)) pr.rho = NAN;
+    prv[0] = pr.rho;
+    prv[1] = pr.vx;
+    prv[2] = pr.vy;
+    prv[3] = pr.vz;
+    prv[4] = pr.p;
   }
-  if (predict_cell(uo, uc, r, O.u_gamma, O.u_rho_floor, O.u_p_floor, up)) {
+  if (first != 0ULL) return;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (!in[d]) continue;
+    S.Pp[d][c] = phi[2 * d];
+    S.BN[d][c] = bn[d];
+    if (wb) B32.BN[d][cb] = (float)bn[d];
+  }
+  if (!cell) return;
+  if (!ok) {
     fail(st, kStagePredict, 0, f, i, j, k);
     return;
   }
-#pragma unroll
-  for (int m = 0; m < 5; ++m) S.Up[m][c] = up[m];
-  Prim pr;
-  if (cons_to_prim(up, O.s_gamma, O.s_rho_floor, O.s_p_floor, &pr)) pr.rho = NAN;
-  const double prv[5] = {pr.rho, pr.vx, pr.vy, pr.vz, pr.p};
+  if (!recovered) fail(st, kStageRecoverPredict, 0, f, i, j, k);
+  const double rho = fmax(up[0], O.e_rho_floor);
 #pragma unroll
   for (int m = 0; m < 5; ++m) {
+    S.Up[m][c] = up[m];
     S.Pr[m][c] = prv[m];
     if (wb) B32.Pr[m][cb] = (float)prv[m];
   }
-  const double v = G.vol[c];
-  const double rho = fmax(up[0], O.e_rho_floor);
 #pragma unroll
   for (int m = 0; m < 3; ++m) {
     const double w = v * up[1 + m] / rho;
     S.W[m][c] = w;
-    if (wb) B32.W[m][cb] = (float)w;
-  }
-  double phi[6];
-#pragma unroll
-  for (int d = 0; d < 3; ++d) {
-    const long long u = c + D.stride(d);
-    phi[2 * d] = S.P[d][c] + r * (S.P[d][c] - S.Po[d][c]);
-    phi[2 * d + 1] = S.P[d][u] + r * (S.P[d][u] - S.Po[d][u]);
-  }
-  double bp[3];
-  if (!recover_cell(G, c, phi, bp)) {
-    fail(st, kStageRecoverPredict, 0, f, i, j, k);
-    return;
-  }
-#pragma unroll
-  for (int m = 0; m < 3; ++m) {
     S.Bp[m][c] = bp[m];
-    if (wb) B32.Bp[m][cb] = (float)bp[m];
+    if (wb) {
+      B32.W[m][cb] = (float)w;
+      B32.Bp[m][cb] = (float)bp[m];
+    }
   }
 }
 #endif  // GCS_SWEEPS_TEMPLATES_ONLY
@@ -117,8 +142,8 @@ __global__ void k_predict(Dims D, DevState S, DevGeom G, Bulk<float> B32, int bu
 // sweeps at 6 x 96x96x192.
 template <typename T>
 struct SweepOccupancy {
-  static constexpr int flux = 4;
-  static constexpr int edge = 6;
+  static constexpr int flux = GCS_FLUX_BLOCKS;
+  static constexpr int edge = GCS_EDGE_BLOCKS;
 };
 template <>
 struct SweepOccupancy<float> {
@@ -127,120 +152,25 @@ struct SweepOccupancy<float> {
 };
 
 // ---------------------------------------------------------------------------
-// Face-flux sweep in direction d (nonorthogonal_sweep.c:408-548).
+// Face-flux sweep, all three directions (nonorthogonal_sweep.c:408-548).
 // Each thread owns one face; the eight-cell stencil of one variable at a
-// time is read from the predictor's cell primitives, so only the volumes,
-// one stencil and the reconstructed face states are live at once.
-template <int d, typename T>
-__global__ void __launch_bounds__(128, SweepOccupancy<T>::flux) k_flux(Dims D, DevState S, Bulk<T> B,
-                                                 Opts O, DevStatus *st, int i0,
-                                                 int i1) {
-  if (failed(st)) return;
+// time is read from the predictor's cell primitives (face_flux,
+// gcs_face_flux.cuh).
+// Bound: FP64 issue and latency at 16 warps an SM (128 registers; 3 to 5
+// blocks of 128 measured within 2 %).  All directions in one launch find a
+// layer's cells in L2 (a launch each: 3.81 against 3.67 ms).  6 x 96x96x192:
+// 4.46 -> 3.02 ms a step, 2774 -> 1700 instructions a face.
+template <bool kOrtho, typename T>
+__global__ void __launch_bounds__(128, SweepOccupancy<T>::flux)
+    k_flux(Dims D, DevState S, const __grid_constant__ Bulk<T> B, Opts O, DevStatus *st,
+           const __grid_constant__ Boxes X) {
+  const int group = (int)blockIdx.y / 3, d = (int)blockIdx.y - 3 * group;
   int f, i, j, k;
-  const Box b{i0, D.g, D.g, D.n + (d == 1), D.n + (d == 2), i1};
-  if (!box_coord(b, &f, &i, &j, &k)) return;
-  const long long c = f * D.Nn + D.node(i, j, k);
-  const long long cb = B.at(f, D.node(i, j, k));   // index of the Bulk arrays
-  const long long sd = D.stride(d);
-  const T iv = B.iv[d][cb];
-  if (isnan(iv)) {
-    fail(st, kStageReconstruct, d, f, i, j, k);
-    return;
-  }
-  const T riv = T(1.0) / iv;
-  const T pdm = (T)O.pdm;
-  T vol[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) vol[n] = B.vol[cb + (n - 4) * sd];
-  PrimT<T> st2[2];
-  {
-    T q[8], l, r;
-    bool ok = true;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) {
-      q[n] = B.Pr[0][cb + (n - 4) * sd];
-      ok = ok && !isnan(q[n]);
-    }
-    if (!ok) {
-      fail(st, kStageReconstruct, d, f, i, j, k);
-      return;
-    }
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].rho = l; st2[1].rho = r;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = B.Pr[1][cb + (n - 4) * sd];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vx = l; st2[1].vx = r;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = B.Pr[2][cb + (n - 4) * sd];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vy = l; st2[1].vy = r;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = B.Pr[3][cb + (n - 4) * sd];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].vz = l; st2[1].vz = r;
-#pragma unroll
-    for (int n = 0; n < 8; ++n) q[n] = B.Pr[4][cb + (n - 4) * sd];
-    up7_pdm_rcp(vol, q, riv, pdm, &l, &r);
-    st2[0].p = l; st2[1].p = r;
-  }
-  T mag[2][3] = {{T(0.0), T(0.0), T(0.0)}, {T(0.0), T(0.0), T(0.0)}};
-  if (O.s_mhd) {
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      T q[8];
-#pragma unroll
-      for (int n = 0; n < 8; ++n) q[n] = B.Bp[m][cb + (n - 4) * sd];
-      up7_pdm_rcp(vol, q, riv, pdm, &mag[0][m], &mag[1][m]);
-    }
-  }
-  FaceFrame<T> fr;
-  fr.nx = B.fn[d][0][cb]; fr.ny = B.fn[d][1][cb]; fr.nz = B.fn[d][2][cb];
-  fr.t1x = B.ft1[d][0][cb]; fr.t1y = B.ft1[d][1][cb]; fr.t1z = B.ft1[d][2][cb];
-  fr.t2x = B.ft2[d][0][cb]; fr.t2y = B.ft2[d][1][cb]; fr.t2z = B.ft2[d][2][cb];
-  FluidFlux<T> fl;
-  if (kinetic_fluid_flux(st2, (T)O.s_gamma, fr, &fl)) {
-    fail(st, kStageKineticFluid, d, f, i, j, k);
-    return;
-  }
-  MaxwellFlux<T> mx;
-  mx.m[0] = mx.m[1] = mx.m[2] = T(0.0);
-  if (O.s_mhd) {
-    const T bn = B.BN[d][cb];
-    T b0[3] = {T(0.0), T(0.0), T(0.0)};
-    T b0n = T(0.0);
-    if (O.s_bg) {
-      b0[0] = B.fb0[d][0][cb];
-      b0[1] = B.fb0[d][1][cb];
-      b0[2] = B.fb0[d][2][cb];
-      b0n = B.fb0n[d][cb];
-    }
-    if (kinetic_maxwell_flux(st2, mag, bn, fr, O.s_bg, b0, b0n, O.s_boris, (T)O.s_c,
-                             fl.vn, &mx)) {
-      fail(st, kStageKineticMaxwell, d, f, i, j, k);
-      return;
-    }
-    if (O.hogs)
-      apply_hogs(&fl, &mx, (T)O.hogs_h, (T)O.hogs_m, O.s_boris, (T)O.s_c);
-    if (O.hogs && O.s_boris) {
-      bool applied;
-      T speed;
-      if (emergency_diffusion(&fl, st2, S.Up, c - sd, c, (T)O.s_c, &applied, &speed)) {
-        fail(st, kStageEmergency, d, f, i, j, k);
-        return;
-      }
-      if (applied) {
-        atomicAdd(&st->emergency_count[f], 1ULL);
-        atomicMax(&st->emergency_max_bits[f],
-                  (unsigned long long)__double_as_longlong((double)speed));
-      }
-    }
-  }
-  const T area = B.area[d][cb];
-#pragma unroll
-  for (int m = 0; m < 5; ++m) B.F[d][m][c] = (double)(area * fl.f[m]);
-#pragma unroll
-  for (int m = 0; m < 3; ++m) B.M[d][m][c] = (double)(area * mx.m[m]);
+  if (!box_coord(X.b[d], &f, &i, &j, &k, group)) return;
+  const FaceAt at{f, i, j, k, (unsigned)(f * D.Nn + D.node(i, j, k)),
+                  (unsigned)B.at(f, D.node(i, j, k))};
+  const GlobalStencil<T> cells(B, at.cb, (int)D.stride(d));
+  face_flux<kOrtho, T>(d, cells, D, S, B, O, st, at);
 }
 
 #ifndef GCS_SWEEPS_TEMPLATES_ONLY
@@ -286,83 +216,85 @@ __global__ void k_seam_flux(Dims D, const Seam *seams, DevState S, DevStatus *st
 // central8 of the per-cell weights over central8 of the volumes, for every
 // face the edge velocities of edge family (a+2)%3 read.
 template <int a, typename T>
-__global__ void k_face_velocity(Dims D, Bulk<T> B, DevStatus *st, int i0,
-                                int i1) {
-  if (failed(st)) return;
-  constexpr int e = (a + 2) % 3, bb = (a + 1) % 3;
+__device__ __forceinline__ void velocity_thread(const Dims &D, const Bulk<T> &B,
+                                                DevStatus *st, const Box &b, int group) {
+  const unsigned long long first = failure_word(st);
   int f, x[3];
-  int lo[3], cnt[3];
-  lo[e] = D.g; cnt[e] = D.act(e);
-  lo[a] = D.g; cnt[a] = D.act(a) + 1;
-  lo[bb] = 0; cnt[bb] = D.ext(bb);
-  const Box b{i0, lo[1], lo[2], cnt[1], cnt[2], i1};
-  if (!box_coord(b, &f, &x[0], &x[1], &x[2])) return;
-  const long long c = f * D.Nn + D.node(x[0], x[1], x[2]);
-  const long long cb = B.at(f, D.node(x[0], x[1], x[2]));
-  const long long sa = D.stride(a);
-  const T riv = T(1.0) / B.iv[a][cb];
+  if (!box_coord(b, &f, &x[0], &x[1], &x[2], group)) return;
+  const unsigned c = (unsigned)(f * D.Nn + D.node(x[0], x[1], x[2]));
+  const unsigned cb = (unsigned)B.at(f, D.node(x[0], x[1], x[2]));
+  const LineStencil<a == 2> at(cb, (int)D.stride(a));
+  const T iv = B.iv[a][cb];
+  T w[3][8];
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    T w[8];
+  for (int m = 0; m < 3; ++m) at.load(B.W[m], w[m]);
+  const T riv = Num<T>::rcp(iv);
+  if (first != 0ULL) return;
 #pragma unroll
-    for (int n = 0; n < 8; ++n) w[n] = B.W[m][cb + (n - 4) * sa];
-    B.FV[a][m][c] = (double)(central8(w) * riv);
-  }
+  for (int m = 0; m < 3; ++m) B.FV[a][m][c] = (double)(central8(w[m]) * riv);
+}
+template <typename T>
+__global__ void k_face_velocity(Dims D, Bulk<T> B, DevStatus *st, Boxes X) {
+  const int group = (int)blockIdx.y / 3, a = (int)blockIdx.y - 3 * group;
+  if (a == 0)
+    velocity_thread<0, T>(D, B, st, X.b[0], group);
+  else if (a == 1)
+    velocity_thread<1, T>(D, B, st, X.b[1], group);
+  else
+    velocity_thread<2, T>(D, B, st, X.b[2], group);
 }
 
 // ---------------------------------------------------------------------------
 // Edge EMF sweep of edge family e (nonorthogonal_sweep.c:624-752).
+// Bound: L2 and HBM traffic (225 B an edge from HBM at 4.5 TB/s, 13 TB/s from
+// L2).  The three families run in one launch because they read the same face
+// velocities, areas and fields: 6 x 96x96x192, with the face velocities, 2.40
+// -> 2.11 ms a step, against 3.02 with a launch per family.
 template <int e, typename T>
-__global__ void __launch_bounds__(128, SweepOccupancy<T>::edge) k_edge_emf(Dims D, DevState S, DevGeom G,
-                                                  Bulk<T> B, Opts O,
-                                                  const StepParams *prm,
-                                                  DevStatus *st, int i0,
-                                                  int i1) {
-  if (failed(st)) return;
+__device__ __forceinline__ void edge_thread(const Dims &D, const DevState &S,
+                                            const unsigned char *edge_ok, const Bulk<T> &B,
+                                            const Opts &O, const StepParams *prm,
+                                            DevStatus *st, const Box &b, int group) {
   constexpr int a = (e + 1) % 3, bb = (e + 2) % 3;
+  const unsigned long long first = failure_word(st);
   int f, x[3];
-  int cnt[3];
-  cnt[e] = D.act(e);
-  cnt[a] = D.act(a) + 1;
-  cnt[bb] = D.act(bb) + 1;
-  const Box b{i0, D.g, D.g, cnt[1], cnt[2], i1};
-  if (!box_coord(b, &f, &x[0], &x[1], &x[2])) return;
-  const long long c = f * D.Nn + D.node(x[0], x[1], x[2]);
-  const long long cb = B.at(f, D.node(x[0], x[1], x[2]));
-  const unsigned char ok = G.edge_ok[e][c];
-  if (ok != 0) {
-    fail(st, ok, e, f, x[0], x[1], x[2]);
-    return;
-  }
-  const long long sa = D.stride(a), sb = D.stride(bb);
-  const T pdm = (T)O.e_pdm;
+  if (!box_coord(b, &f, &x[0], &x[1], &x[2], group)) return;
+  const unsigned c = (unsigned)(f * D.Nn + D.node(x[0], x[1], x[2]));
+  const unsigned cb = (unsigned)B.at(f, D.node(x[0], x[1], x[2]));
+  const unsigned char geometry = edge_ok[c];
+  const int sa = (int)D.stride(a), sb = (int)D.stride(bb);
+  const T pdm2 = T(2.0) * (T)O.e_pdm;
   // edge velocity: faces of family a along bb
-  T ar[8], fld[8];
+  T fld[8];
   T v[3];
+  T fl, fr, sl, sr;
+  {
+    const LineStencil<bb == 2> at(cb, sb), full(c, sb);
+    T ar[8];
+    at.load(B.area[a], ar);
+    const T rca = Num<T>::rcp(B.ca[e][cb]);
 #pragma unroll
-  for (int n = 0; n < 8; ++n) ar[n] = B.area[a][cb + (n - 4) * sb];
-  const T rca = T(1.0) / B.ca[e][cb];
+    for (int m = 0; m < 3; ++m) {
+      double fv[8];
+      full.load(B.FV[a][m], fv);
+      T w[8];
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    T w[8];
-#pragma unroll
-    for (int n = 0; n < 8; ++n) w[n] = ar[n] * (T)B.FV[a][m][c + (n - 4) * sb];
-    v[m] = central8(w) * rca;
+      for (int n = 0; n < 8; ++n) w[n] = ar[n] * (T)fv[n];
+      v[m] = central8(w) * rca;
+    }
+    // transverse face fields (nonorthogonal_sweep.c:372-406)
+    at.load(B.BN[a], fld);
+    up7_pdm(Up7Weights<T>(ar, rca), fld, pdm2, &fl, &fr);
   }
   const T vt1 = dot3(v[0], v[1], v[2], B.et1[e][0][cb], B.et1[e][1][cb], B.et1[e][2][cb]);
   const T vt2 = dot3(v[0], v[1], v[2], B.et2[e][0][cb], B.et2[e][1][cb], B.et2[e][2][cb]);
-  // transverse face fields (nonorthogonal_sweep.c:372-406)
-  T fl, fr, sl, sr;
-#pragma unroll
-  for (int n = 0; n < 8; ++n) fld[n] = B.BN[a][cb + (n - 4) * sb];
-  up7_pdm_rcp(ar, fld, rca, pdm, &fl, &fr);
-  T ar2[8];
-#pragma unroll
-  for (int n = 0; n < 8; ++n) {
-    ar2[n] = B.area[bb][cb + (n - 4) * sa];
-    fld[n] = B.BN[bb][cb + (n - 4) * sa];
+  {
+    const LineStencil<a == 2> at(cb, sa);
+    T ar[8];
+    at.load(B.area[bb], ar);
+    at.load(B.BN[bb], fld);
+    up7_pdm(Up7Weights<T>(ar, Num<T>::rcp(B.cb[e][cb])), fld, pdm2, &sl, &sr);
   }
-  up7_pdm_rcp(ar2, fld, T(1.0) / B.cb[e][cb], pdm, &sl, &sr);
   // 2x2 edge solve (nonorthogonal_operators.c:56-79)
   const T f1 = T(0.5) * (fl + fr);
   const T f2 = T(0.5) * (sl + sr);
@@ -377,22 +309,36 @@ __global__ void __launch_bounds__(128, SweepOccupancy<T>::edge) k_edge_emf(Dims 
   }
   const T jump = (sr - sl) - (fr - fl);
   // edge density (nonorthogonal_sweep.c:351-370), from the FP64 state
+  const double *up0 = S.Up[0];
   double rho = 0.0;
-  rho += 0.25 * S.Up[0][c];
-  rho += 0.25 * S.Up[0][c - sb];
-  rho += 0.25 * S.Up[0][c - sa];
-  rho += 0.25 * S.Up[0][c - sa - sb];
-  if (!(isfinite(rho) && rho > DBL_MIN)) {
-    fail(st, kStageEdgeDensity, e, f, x[0], x[1], x[2]);
-    return;
-  }
+  rho += 0.25 * up0[c];
+  rho += 0.25 * up0[c - (unsigned)sb];
+  rho += 0.25 * up0[c - (unsigned)sa];
+  rho += 0.25 * up0[c - (unsigned)(sa + sb)];
+  const bool rho_ok = isfinite(rho) && rho > DBL_MIN;
   T emf;
-  if (edge_emf(vt1, vt2, ef0, ef1, jump, (T)rho, B.elen[e][cb], (T)O.e_diff, O.e_boris,
-               (T)O.e_c, (T)O.e_cfl, (T)prm->dt, &emf)) {
-    fail(st, kStageEdgeEmf, e, f, x[0], x[1], x[2]);
+  const bool emf_ok =
+      edge_emf(vt1, vt2, ef0, ef1, jump, (T)rho, B.elen[e][cb], (T)O.e_diff, O.e_boris,
+               (T)O.e_c, (T)(O.e_cfl * Num<double>::rcp(prm->dt)), &emf) == 0;
+  if (first != 0ULL) return;
+  if (geometry != 0 || !rho_ok || !emf_ok) {
+    fail(st, geometry != 0 ? geometry : !rho_ok ? kStageEdgeDensity : kStageEdgeEmf, e, f,
+         x[0], x[1], x[2]);
     return;
   }
   B.E[e][c] = (double)emf;
+}
+template <typename T>
+__global__ void __launch_bounds__(128, SweepOccupancy<T>::edge)
+    k_edge_emf(Dims D, DevState S, DevGeom G, Bulk<T> B, Opts O, const StepParams *prm,
+               DevStatus *st, Boxes X) {
+  const int group = (int)blockIdx.y / 3, e = (int)blockIdx.y - 3 * group;
+  if (e == 0)
+    edge_thread<0, T>(D, S, G.edge_ok[0], B, O, prm, st, X.b[0], group);
+  else if (e == 1)
+    edge_thread<1, T>(D, S, G.edge_ok[1], B, O, prm, st, X.b[1], group);
+  else
+    edge_thread<2, T>(D, S, G.edge_ok[2], B, O, prm, st, X.b[2], group);
 }
 
 #ifndef GCS_SWEEPS_TEMPLATES_ONLY
@@ -419,116 +365,155 @@ __global__ void k_edge_sync(Dims D, const int *offsets, const EdgeMember *mem,
 
 // ---------------------------------------------------------------------------
 // Save Phi -> Phi_old on every face, then the CT curl on active faces
-// (nonorthogonal_step.c:233-298, 361-377).
-template <int d>
-__global__ void k_ct(Dims D, DevState S, Opts O, const StepParams *prm, DevStatus *st) {
-  if (failed(st)) return;
-  int f, i, j, k;
-  const Box b{0, 0, 0, D.E1 + (d == 1), D.E2 + (d == 2), D.E0 + (d == 0)};
-  if (!box_coord(b, &f, &i, &j, &k)) return;
-  const long long c = f * D.Nn + D.node(i, j, k);
-  const double old = S.P[d][c];
-  S.Po[d][c] = old;
-  if (!O.u_mhd) return;
-  const int x[3] = {i, j, k};
+// (nonorthogonal_step.c:233-298, 361-377): the three faces of a node share
+// its edge EMFs, nine reads where a launch per family makes twelve.  families:
+// bit per face family of the launch.
+__global__ void k_ct(Dims D, DevState S, Opts O, int families, const StepParams *prm,
+                     DevStatus *st) {
+  const unsigned long long first = failure_word(st);
+  int f, x[3];
+  const Box b{0, 0, 0, D.E1 + 1, D.E2 + 1, D.E0 + 1};
+  if (!box_coord(b, &f, &x[0], &x[1], &x[2])) return;
+  const unsigned c = (unsigned)(f * D.Nn + D.node(x[0], x[1], x[2]));
+  const unsigned s0 = (unsigned)D.stride(0), s1 = (unsigned)D.stride(1);
+  bool in[3], active[3];
+  double old[3], curl[3] = {0.0, 0.0, 0.0};
 #pragma unroll
-  for (int a = 0; a < 3; ++a)
-    if (x[a] < D.g || x[a] >= D.g + D.act(a) + (a == d)) return;
-  const long long s0 = D.stride(0), s1 = D.stride(1);
+  for (int d = 0; d < 3; ++d) {
+    in[d] = families >> d & 1;
+    active[d] = in[d] && O.u_mhd;
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+      in[d] = in[d] && x[a] < D.ext(a) + (a == d);
+      active[d] = active[d] && x[a] >= D.g && x[a] < D.g + D.act(a) + (a == d);
+    }
+    old[d] = in[d] ? S.P[d][c] : 0.0;
+  }
   double *const *E = S.E;
-  double curl;
-  if (d == 0)
-    curl = E[2][c + s1] - E[2][c] - E[1][c + 1] + E[1][c];
-  else if (d == 1)
-    curl = E[0][c + 1] - E[0][c] - E[2][c + s0] + E[2][c];
-  else
-    curl = E[1][c + s0] - E[1][c] - E[0][c + s1] + E[0][c];
-  S.P[d][c] = old - prm->dt * curl;
+  if (active[0] || active[1] || active[2]) {
+    // edge reads of an inactive face of the node stay inside the arrays
+    const double e0 = E[0][c], e1 = E[1][c], e2 = E[2][c];
+    if (active[0]) curl[0] = E[2][c + s1] - e2 - E[1][c + 1] + e1;
+    if (active[1]) curl[1] = E[0][c + 1] - e0 - E[2][c + s0] + e2;
+    if (active[2]) curl[2] = E[1][c + s0] - e1 - E[0][c + s1] + e0;
+  }
+  const double dt = prm->dt;
+  if (first != 0ULL) return;
+#pragma unroll
+  for (int d = 0; d < 3; ++d) {
+    if (in[d]) S.Po[d][c] = old[d];
+    if (active[d]) S.P[d][c] = old[d] - dt * curl[d];
+  }
 }
 
 // Cell update (nonorthogonal_step.c:527-610 with the stress rates of
-// nonorthogonal_sweep.c:550-622): save U, B as old on every cell, then on
-// active cells U += dt * rate, recover B from the CT-updated Phi, and apply
-// the Boris (nonorthogonal_state.c:161-280) or Maxwell momentum update.
-__global__ void __launch_bounds__(128, 6) k_update(Dims D, DevState S, DevGeom G,
-                                                DevBg BG, Opts O,
+// nonorthogonal_sweep.c:550-622) and final recovery (cubedsphere_step.c:
+// 142-152) of every cell: save U, B as old, on active cells U += dt * rate,
+// recover B from the CT-updated Phi, apply the Boris (nonorthogonal_state.c:
+// 161-280) or Maxwell momentum update, store B; in driver mode the CFL time
+// step of the new state (nonorthogonal_step.c:449-525).
+//
+// The reference recovers B before the seam sync of Phi for the momentum
+// update and again after it on every cell.  The two sides of a seam face
+// carry the same synced Phi and edge EMFs, so the sync moves Phi by the
+// rounding of the curl only; here it runs before this kernel and one
+// recovery serves both uses, which saves a second pass over the recovery
+// map, Phi, U and B0 (264 B per cell).  Bound: HBM (4.9 TB/s).  Four blocks an
+// SM (124 registers): at six, the bound without the recovery, it spills.
+// 6 x 96x96x192, CT, update and recovery: 2.72 -> 1.79 ms a step (six blocks
+// 2.21, five 1.99).
+__global__ void __launch_bounds__(128, GCS_UPDATE_BLOCKS) k_update(Dims D, DevState S, DevGeom G,
+                                                DevBg BG, Opts O, int with_cfl,
                                                 const StepParams *prm,
                                                 DevStatus *st) {
-  if (failed(st)) return;
+  const unsigned long long first = failure_word(st);
   int f, i, j, k;
   const Box b{0, 0, 0, D.E1, D.E2, D.E0};
-  if (!box_coord(b, &f, &i, &j, &k)) return;
-  const long long c = f * D.Nn + D.node(i, j, k);
-  double u[5], bo[3];
+  double cand = DBL_MAX;
+  if (box_coord(b, &f, &i, &j, &k)) {
+    const unsigned c = (unsigned)(f * D.Nn + D.node(i, j, k));
+    const unsigned sdir[3] = {(unsigned)D.stride(0), (unsigned)D.stride(1), 1u};
+    const bool active = i >= D.g && i < D.g + D.nr && j >= D.g && j < D.g + D.n &&
+                        k >= D.g && k < D.g + D.n;
+    double uold[5], bo[3], bn[3] = {0.0, 0.0, 0.0}, b0[3] = {0.0, 0.0, 0.0};
+    bool recovered = true;
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    u[m] = S.U[m][c];
-    S.Uo[m][c] = u[m];
-  }
+    for (int m = 0; m < 5; ++m) uold[m] = S.U[m][c];
 #pragma unroll
-  for (int m = 0; m < 3; ++m) {
-    bo[m] = S.B[m][c];
-    S.Bo[m][c] = bo[m];
-  }
-  if (i < D.g || i >= D.g + D.nr || j < D.g || j >= D.g + D.n || k < D.g ||
-      k >= D.g + D.n)
-    return;
-  const double dt = prm->dt;
-  const double iv = G.ivol[c];
-  double rate[5], mrate[3];
-  const long long sdir[3] = {D.stride(0), D.stride(1), 1};
+    for (int m = 0; m < 3; ++m) bo[m] = S.B[m][c];
+    if (O.u_mhd) {
+      double phi[6];
 #pragma unroll
-  for (int m = 0; m < 5; ++m) {
-    double diff = 0.0;
-#pragma unroll
-    for (int d = 0; d < 3; ++d) diff += S.F[d][m][c] - S.F[d][m][c + sdir[d]];
-    rate[m] = diff * iv;
-  }
-  const double uold[5] = {u[0], u[1], u[2], u[3], u[4]};
-#pragma unroll
-  for (int m = 0; m < 5; ++m) u[m] += dt * rate[m];
-  if (O.u_mhd) {
-#pragma unroll
-    for (int m = 0; m < 3; ++m) {
-      double diff = 0.0;
-#pragma unroll
-      for (int d = 0; d < 3; ++d)
-        diff += S.M[d][m][c] - S.M[d][m][c + sdir[d]];
-      mrate[m] = diff * iv;
-      if (O.u_bg) mrate[m] += BG.force[m][c];
+      for (int d = 0; d < 3; ++d) {
+        phi[2 * d] = S.P[d][c];
+        phi[2 * d + 1] = S.P[d][c + sdir[d]];
+      }
+      recovered = recover_cell(G, c, phi, bn);
     }
-    double phi[6], bn[3];
+    double u[5];
+    int code = recovered ? kStageNone : active ? kStageRecoverUpdate : kStageRecoverFinal;
+    if (active) {
+      const double dt = prm->dt;
+      const double iv = G.ivol[c];
+      double rate[5], mrate[3];
 #pragma unroll
-    for (int d = 0; d < 3; ++d) {
-      phi[2 * d] = S.P[d][c];
-      phi[2 * d + 1] = S.P[d][c + sdir[d]];
-    }
-    if (!recover_cell(G, c, phi, bn)) {
-      fail(st, kStageRecoverUpdate, 0, f, i, j, k);
-      return;
-    }
-    if (O.u_boris) {
-      double nb[3] = {bn[0], bn[1], bn[2]};
-      double ob[3] = {bo[0], bo[1], bo[2]};
-      if (O.u_bg) {
+      for (int m = 0; m < 5; ++m) {
+        double diff = 0.0;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) diff += S.F[d][m][c] - S.F[d][m][c + sdir[d]];
+        rate[m] = diff * iv;
+        u[m] = uold[m] + dt * rate[m];
+      }
+      if (O.u_mhd) {
 #pragma unroll
         for (int m = 0; m < 3; ++m) {
-          const double b0 = BG.b0[m][c];
-          nb[m] = bn[m] + b0;
-          ob[m] = bo[m] + b0;
+          double diff = 0.0;
+#pragma unroll
+          for (int d = 0; d < 3; ++d)
+            diff += S.M[d][m][c] - S.M[d][m][c + sdir[d]];
+          mrate[m] = diff * iv;
+          if (O.u_bg) mrate[m] += BG.force[m][c];
+          if (O.u_bg || (with_cfl && O.t_bg)) b0[m] = BG.b0[m][c];
+        }
+        if (O.u_boris) {
+          double nb[3], ob[3];
+#pragma unroll
+          for (int m = 0; m < 3; ++m) {
+            nb[m] = O.u_bg ? bn[m] + b0[m] : bn[m];
+            ob[m] = O.u_bg ? bo[m] + b0[m] : bo[m];
+          }
+          if (apply_boris(u, uold, nb, ob, rate, mrate, O.u_c, dt, O.u_gamma,
+                          O.u_rho_floor, O.u_p_floor) &&
+              code == kStageNone)
+            code = kStageUpdate;
+        } else {
+          apply_maxwell(u, mrate, dt, O.u_gamma, O.u_rho_floor, O.u_p_floor);
         }
       }
-      if (apply_boris(u, uold, nb, ob, rate, mrate, O.u_c, dt, O.u_gamma,
-                      O.u_rho_floor, O.u_p_floor)) {
-        fail(st, kStageUpdate, 0, f, i, j, k);
-        return;
+    }
+    if (first == 0ULL) {
+#pragma unroll
+      for (int m = 0; m < 5; ++m) S.Uo[m][c] = uold[m];
+#pragma unroll
+      for (int m = 0; m < 3; ++m) S.Bo[m][c] = bo[m];
+      if (code != kStageNone) {
+        fail(st, code, 0, f, i, j, k);
+      } else {
+        if (active) {
+#pragma unroll
+          for (int m = 0; m < 5; ++m) S.U[m][c] = u[m];
+        }
+        if (O.u_mhd) {
+#pragma unroll
+          for (int m = 0; m < 3; ++m) S.B[m][c] = bn[m];
+          if (with_cfl && active && !cfl_step(O, u, bn, b0, G.cflmin[c], &cand))
+            fail(st, kStageTimestep, 0, f, i, j, k);
+        }
       }
-    } else {
-      apply_maxwell(u, mrate, dt, O.u_gamma, O.u_rho_floor, O.u_p_floor);
     }
   }
-#pragma unroll
-  for (int m = 0; m < 5; ++m) S.U[m][c] = u[m];
+  // every thread of the block reaches the reduction
+  if (with_cfl) reduce_cfl(cand, st);
 }
 
 #endif  // GCS_SWEEPS_TEMPLATES_ONLY
@@ -545,13 +530,50 @@ inline bool clamp_range(int lo, int hi, int i0, int i1, int *a, int *n) {
   return *n > 0;
 }
 
+// Layer range of each family of a sweep over [i0, i1): family q covers
+// [lo[q], hi[q]).  Returns the layer groups of the launch (0: nothing to do);
+// an empty family has no points.
+inline int clamp_boxes(Boxes &X, const int lo[3], const int hi[3], int i0, int i1, Tile t) {
+  int groups = 0;
+  for (int q = 0; q < 3; ++q) {
+    int a = 0, n = 0;
+    if (!clamp_range(lo[q], hi[q], i0, i1, &a, &n)) n = 0;
+    X.b[q].i0 = a;
+    X.b[q].i1 = a + n;
+    const int g = (n + t.by - 1) / t.by;
+    groups = g > groups ? g : groups;
+  }
+  return groups;
+}
+inline dim3 boxes_grid(const Boxes &X, int groups, Tile t) {
+  int points = 0;
+  for (int q = 0; q < 3; ++q) points = max(points, X.b[q].nj * X.b[q].nk);
+  return dim3((unsigned)((points + t.bx - 1) / t.bx), 3u * (unsigned)groups, kFaces);
+}
+// A sweep's launches over [i0, i1): all families at once, or one at a time
+// (Ctx::split_families).
+template <typename Launch>
+void launch_families(const Ctx &X, Boxes b, const int lo[3], const int hi[3], int i0, int i1,
+                     Tile t, Launch launch) {
+  for (int only = X.split_families ? 0 : -1; only < (X.split_families ? 3 : 0); ++only) {
+    int l[3], h[3];
+    for (int q = 0; q < 3; ++q) {
+      const bool on = only < 0 || q == only;
+      l[q] = on ? lo[q] : 0;
+      h[q] = on ? hi[q] : 0;
+    }
+    const int groups = clamp_boxes(b, l, h, i0, i1, t);
+    if (groups > 0) launch(boxes_grid(b, groups, t), b);
+  }
+}
+
 template <typename T>
 struct Sweeps {
   static void flux(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                    cudaStream_t s) {
     const Dims &D = X.D;
-    int a, n;
     if (X.flux_staged) {
+      int a, n;
       if (clamp_range(D.g, D.g + D.nr + 1, i0, i1, &a, &n))
         launch_flux_tma<0, T>(X, B, O, a, a + n, s);
       if (clamp_range(D.g, D.g + D.nr, i0, i1, &a, &n))
@@ -561,46 +583,53 @@ struct Sweeps {
       return;
     }
     const Tile t = X.tile[kTileFlux];
-    if (clamp_range(D.g, D.g + D.nr + 1, i0, i1, &a, &n))
-      k_flux<0, T><<<tile_grid(n, D.n, D.n, t), tile_block(t), 0, s>>>(
-          D, X.S, B, O, X.status, a, a + n);
-    if (clamp_range(D.g, D.g + D.nr, i0, i1, &a, &n))
-      k_flux<1, T><<<tile_grid(n, D.n + 1, D.n, t), tile_block(t), 0, s>>>(
-          D, X.S, B, O, X.status, a, a + n);
-    if (clamp_range(D.g, D.g + D.nr, i0, i1, &a, &n))
-      k_flux<2, T><<<tile_grid(n, D.n, D.n + 1, t), tile_block(t), 0, s>>>(
-          D, X.S, B, O, X.status, a, a + n);
+    Boxes b;
+    for (int d = 0; d < 3; ++d)
+      b.b[d] = Box{0, D.g, D.g, D.n + (d == 1), D.n + (d == 2), 0};
+    const int lo[3] = {D.g, D.g, D.g}, hi[3] = {D.g + D.nr + 1, D.g + D.nr, D.g + D.nr};
+    // FP32 reads the tangents: its rounded frame is not orthonormal to FP32
+    const bool ortho = X.ortho && sizeof(T) == 8;
+    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
+      (ortho ? k_flux<true, T> : k_flux<false, T>)
+          <<<grid, tile_block(t), 0, s>>>(D, X.S, B, O, X.status, boxes);
+    });
   }
   static void emf(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                   cudaStream_t s) {
     const Dims &D = X.D;
-    int a, n;
     // face velocities: family a, edge family e=(a+2)%3 active, a faces, bb all
     const Tile t = X.tile[kTileFaceVelocity];
-    if (clamp_range(D.g, D.g + D.nr + 1, i0, i1, &a, &n))  // e=2, a=0, bb=1
-      k_face_velocity<0, T><<<tile_grid(n, D.E1, D.n, t), tile_block(t), 0, s>>>(
-          D, B, X.status, a, a + n);
-    if (clamp_range(D.g, D.g + D.nr, i0, i1, &a, &n))  // e=0, a=1, bb=2
-      k_face_velocity<1, T><<<tile_grid(n, D.n + 1, D.E2, t), tile_block(t), 0, s>>>(
-          D, B, X.status, a, a + n);
-    if (clamp_range(0, D.E0, i0, i1, &a, &n))  // e=1, a=2, bb=0 (all i)
-      k_face_velocity<2, T><<<tile_grid(n, D.n, D.n + 1, t), tile_block(t), 0, s>>>(
-          D, B, X.status, a, a + n);
+    Boxes b;
+    int lo[3], hi[3];
+    for (int a = 0; a < 3; ++a) {
+      const int e = (a + 2) % 3, bb = (a + 1) % 3;
+      int first[3], count[3];
+      first[e] = D.g; count[e] = D.act(e);
+      first[a] = D.g; count[a] = D.act(a) + 1;
+      first[bb] = 0; count[bb] = D.ext(bb);
+      lo[a] = first[0];
+      hi[a] = first[0] + count[0];
+      b.b[a] = Box{0, first[1], first[2], count[1], count[2], 0};
+    }
+    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
+      k_face_velocity<T><<<grid, tile_block(t), 0, s>>>(D, B, X.status, boxes);
+    });
   }
   static void edge(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                    cudaStream_t s) {
     const Dims &D = X.D;
-    int a, n;
     const Tile t = X.tile[kTileEdgeEmf];
-    if (clamp_range(D.g, D.g + D.nr, i0, i1, &a, &n))
-      k_edge_emf<0, T><<<tile_grid(n, D.n + 1, D.n + 1, t), tile_block(t), 0, s>>>(
-          D, X.S, X.G, B, O, X.params, X.status, a, a + n);
-    if (clamp_range(D.g, D.g + D.nr + 1, i0, i1, &a, &n))
-      k_edge_emf<1, T><<<tile_grid(n, D.n, D.n + 1, t), tile_block(t), 0, s>>>(
-          D, X.S, X.G, B, O, X.params, X.status, a, a + n);
-    if (clamp_range(D.g, D.g + D.nr + 1, i0, i1, &a, &n))
-      k_edge_emf<2, T><<<tile_grid(n, D.n + 1, D.n, t), tile_block(t), 0, s>>>(
-          D, X.S, X.G, B, O, X.params, X.status, a, a + n);
+    Boxes b;
+    int lo[3], hi[3];
+    for (int e = 0; e < 3; ++e) {
+      lo[e] = D.g;
+      hi[e] = D.g + D.nr + (e != 0);
+      b.b[e] = Box{0, D.g, D.g, D.n + (e != 1), D.n + (e != 2), 0};
+    }
+    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
+      k_edge_emf<T><<<grid, tile_block(t), 0, s>>>(D, X.S, X.G, B, O, X.params, X.status,
+                                                   boxes);
+    });
   }
 };
 

@@ -1,0 +1,117 @@
+"""The forms of the step's sweeps and transfers that a plain case does not
+reach: face frames that are not orthonormal (the flux sweep then reads the
+tangents), one launch per family, and state transfers at sizes that leave
+partial blocks."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from gamera_cube_b200 import abi
+from gamera_cube_b200.host import HostStorage
+from oracle import oracle_cases
+from tests.parity_util import compare_state
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def lib():
+    import gamera_cube_b200
+    return gamera_cube_b200.lib
+
+
+def scale_tangents(case, factor):
+    """Tangents of every face times `factor`: the flux projects on them and
+    back, so the momentum flux along them scales by factor^2."""
+    for f in range(6):
+        grid = case.grid[f]
+        for d in range(3):
+            faces = grid.face[d]
+            count = faces.extent[0] * faces.extent[1] * faces.extent[2]
+            at = C.cast(faces.value, C.POINTER(C.c_double))
+            view = np.ctypeslib.as_array(at, shape=(count, C.sizeof(abi.FaceGeometry) // 8))
+            first = abi.FaceGeometry.tangent1.offset // 8
+            view[:, first:first + 6] *= factor
+
+
+@pytest.mark.parametrize("factor", [1.0, 1.0 + 1e-7, 0.9])
+@pytest.mark.parametrize("kind,nr,n", [("wind", 12, 9), ("shock", 17, 11)])
+def test_frames(lib, kind, nr, n, factor):
+    """One step against the restatement on the same grid: 1e-12 normwise,
+    orthonormal frames (factor 1) or not.  1e-7 off shows a sweep that took
+    the orthonormal form on a frame that is not: the momentum flux along the
+    tangents would be 2e-7 off."""
+    ref, gpu = oracle_cases.pair(kind, nr, n, 5)
+    scale_tangents(ref, factor)
+    scale_tangents(gpu, factor)
+    plan = C.c_void_p()
+    assert lib.gamera_cs_halo_plan_create(gpu.grid, gpu.active, gpu.ghost,
+                                          C.byref(plan)) == 0, lib.gcs_last_error()
+    try:
+        dt = 0.4 * ref.local_timestep()
+        assert ref.step(0.0, dt) == 0
+        assert lib.gamera_cs_advance_six_with_background_planned(
+            gpu.grid, gpu.storage, gpu.active, gpu.ghost, 0.0, dt, gpu.options,
+            gpu.background, plan, None, 0.0, 0.0, None) == 0
+        bad = {k: v for k, v in compare_state(gpu, ref).items() if not v[0] <= 1e-12}
+        assert not bad, bad
+    finally:
+        lib.gamera_cs_halo_plan_destroy(plan)
+
+
+@pytest.mark.parametrize("bulk", [0, 1])
+def test_one_launch_per_family(lib, bulk):
+    """A run of an ensemble (one launch per face and edge family) and the
+    same run stepped alone (all families in a launch) agree bit for bit."""
+    driver = abi.WindDriver(7.0, -420.0, 9e4, -4.0)
+    nr, n = (C.c_size_t * 1)(26), (C.c_size_t * 1)(11)
+    config = abi.EnsembleConfig()
+    config.count, config.nr, config.n = 1, nr, n
+    config.drivers = C.pointer(driver)
+    config.seed, config.fp32_bulk, config.dt_fraction = 3, bulk, 0.5
+    e = lib.gcs_ensemble_create(C.byref(config))
+    assert e, lib.gcs_last_error()
+    alone = lib.gcs_context_create_wind(26, 11, 3, C.byref(driver))
+    assert alone
+    try:
+        if bulk:
+            assert lib.gcs_context_set_precision(alone, 1) == 0
+        o, t = abi.AdvanceOptions(), abi.TimestepOptions()
+        lib.gcs_case_options(2, C.byref(o), C.byref(t))
+        bad = C.c_int()
+        assert lib.gcs_ensemble_advance(e, 4) == 0
+        assert lib.gcs_ensemble_sync(e, C.byref(bad)) == 0
+        assert lib.gcs_context_run(alone, C.byref(o), C.byref(t), 0.5, 4, 1) == 0
+        assert lib.gcs_context_sync(alone) == 0
+        a, b = HostStorage([26, 11, 11], 4), HostStorage([26, 11, 11], 4)
+        assert lib.gcs_context_download_state(lib.gcs_ensemble_run_context(e, 0),
+                                              a.storage, 0) == 0
+        assert lib.gcs_context_download_state(alone, b.storage, 0) == 0
+        for f in range(6):
+            x, y = a.arrays(f), b.arrays(f)
+            for name in x:
+                np.testing.assert_array_equal(x[name], y[name], err_msg=name)
+    finally:
+        lib.gcs_context_destroy(alone)
+        lib.gcs_ensemble_destroy(e)
+
+
+@pytest.mark.parametrize("nr,n,pinned", [(9, 9, False), (13, 10, True), (31, 17, False)])
+def test_state_round_trip(lib, nr, n, pinned):
+    """Random state arrays, uploaded and downloaded, come back bit for bit."""
+    ctx = lib.gcs_context_create_case(1, nr, n, 1)
+    assert ctx, lib.gcs_last_error()
+    try:
+        a = HostStorage([nr, n, n], 4, pinned=pinned, scratch=False)
+        b = HostStorage([nr, n, n], 4, pinned=pinned, scratch=False)
+        rng = np.random.default_rng(nr)
+        for q in a._keep:
+            np.asarray(q)[:] = rng.standard_normal(len(q))
+        assert lib.gcs_context_upload_state(ctx, a.storage) == 0
+        assert lib.gcs_context_download_state(ctx, b.storage, 0) == 0
+        for x, y in zip(a._keep, b._keep):
+            np.testing.assert_array_equal(np.asarray(x), np.asarray(y))
+    finally:
+        lib.gcs_context_destroy(ctx)
+
