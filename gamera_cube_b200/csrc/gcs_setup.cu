@@ -341,6 +341,38 @@ __global__ void k_gather(Dims D, int f, int e0, int e1, int e2, int ncomp,
   for (int q = 0; q < ncomp; ++q) dst[t * ncomp + q] = src.p[q][c];
 }
 
+// The ten state arrays of one face in the reference layout, one after the
+// other in a staging buffer (U, U_old, B, B_old, then Phi and Phi_old of each
+// face family): array a has comps[a] device arrays and extents e[a], and
+// starts at start[a].
+struct StateArrays {
+  double *p[10][5];
+  int comps[10], e[10][3];
+  long long start[10], count[10];
+};
+
+// Staging to device arrays (upload) or back, one launch per face: a thread
+// per point and array.
+template <bool kUpload>
+__global__ void k_move_state(Dims D, int f, StateArrays A, double *stage) {
+  const int a = blockIdx.y;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= A.count[a]) return;
+  const int e1 = A.e[a][1], e2 = A.e[a][2];
+  const int k = (int)(t % e2), j = (int)((t / e2) % e1), i = (int)(t / ((long long)e1 * e2));
+  const long long c = f * D.Nn + D.node(i, j, k);
+  const int n = A.comps[a];
+  double *s = stage + A.start[a] + t * n;
+#pragma unroll
+  for (int q = 0; q < 5; ++q) {
+    if (q >= n) break;
+    if (kUpload)
+      A.p[a][q][c] = s[q];
+    else
+      s[q] = A.p[a][q][c];
+  }
+}
+
 }  // namespace
 
 // ---------------------------------------------------------------------------
@@ -830,37 +862,86 @@ int Context::transfer_array(int f, int kind, int dir, bool upload, double *host)
   return 0;
 }
 
-int Context::upload_state(const gamera_no_storage st[kFaces]) {
+// Moves the state arrays of all faces between the caller's host arrays and
+// the device: per face one gather or scatter kernel and one copy per array,
+// all queued on the context's stream, the faces cycling through as many
+// staging slots as fit, and one wait at the end.  Bound: the host link, and
+// the copies' starts on small grids.  With a wait after every array the
+// drop-in step of 6 x 32x32x48 took 6.3 ms, now 4.5 (95 MB each way); four
+// steps of 6 x 9x9x12 with one download 1.96 ms, now 0.94.
+int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
+  const Dims &D = X.D;
+  StateArrays A{};
+  long long total = 0, most = 0;
+  auto add = [&](int a, double *const *p, int comps, int dir) {
+    A.comps[a] = comps;
+    A.count[a] = 1;
+    for (int x = 0; x < 3; ++x) {
+      A.e[a][x] = D.ext(x) + (x == dir);
+      A.count[a] *= A.e[a][x];
+    }
+    for (int q = 0; q < comps; ++q) A.p[a][q] = p[q];
+    A.start[a] = total;
+    total += A.count[a] * comps;
+    most = std::max(most, A.count[a]);
+  };
+  add(0, X.S.U, 5, -1);
+  add(1, X.S.Uo, 5, -1);
+  add(2, X.S.B, 3, -1);
+  add(3, X.S.Bo, 3, -1);
+  for (int d = 0; d < 3; ++d) {
+    add(4 + 2 * d, &X.S.P[d], 1, d);
+    add(5 + 2 * d, &X.S.Po[d], 1, d);
+  }
+  const size_t bytes = (size_t)total * sizeof(double);
+  if (owner && staging_bytes < bytes) {
+    // runs sharing a grid allocate their transfer buffer on first use
+    if (staging) GCS_TRY(cudaFree(staging));
+    staging = nullptr;
+    staging_bytes = 0;
+    GCS_TRY(cudaMalloc(&staging, bytes));
+    staging_bytes = bytes;
+  }
+  const int slots = (int)std::min<size_t>(kFaces, staging_bytes / bytes);
+  if (slots < 1) {
+    set_error("staging too small", "transfer");
+    return -1;
+  }
+  const dim3 grid(blocks_for(most, 256), 10);
   for (int f = 0; f < kFaces; ++f) {
+    double *stage = (double *)staging + (long long)(f % slots) * total;
+    double *host[10] = {st[f].conserved, st[f].old_conserved, (double *)st[f].cell_magnetic,
+                        (double *)st[f].old_cell_magnetic,
+                        st[f].face_flux[0], st[f].old_face_flux[0],
+                        st[f].face_flux[1], st[f].old_face_flux[1],
+                        st[f].face_flux[2], st[f].old_face_flux[2]};
+    if (!upload) k_move_state<false><<<grid, 256, 0, stream>>>(D, f, A, stage);
+    for (int a = 0; a < 10; ++a) {
+      const size_t n = (size_t)A.count[a] * A.comps[a] * sizeof(double);
+      double *s = stage + A.start[a];
+      GCS_TRY(upload ? cudaMemcpyAsync(s, host[a], n, cudaMemcpyHostToDevice, stream)
+                     : cudaMemcpyAsync(host[a], s, n, cudaMemcpyDeviceToHost, stream));
+    }
+    if (upload) k_move_state<true><<<grid, 256, 0, stream>>>(D, f, A, stage);
+  }
+  GCS_TRY(cudaGetLastError());
+  GCS_TRY(cudaStreamSynchronize(stream));
+  return 0;
+}
+
+int Context::upload_state(const gamera_no_storage st[kFaces]) {
+  for (int f = 0; f < kFaces; ++f)
     for (int a = 0; a < 3; ++a)
       if (st[f].cell_extent[a] != (size_t)X.D.ext(a)) {
         set_error("storage extent mismatch", "upload_state");
         return -1;
       }
-    if (transfer_array(f, kArrU, 0, true, st[f].conserved) ||
-        transfer_array(f, kArrUo, 0, true, st[f].old_conserved) ||
-        transfer_array(f, kArrB, 0, true, (double *)st[f].cell_magnetic) ||
-        transfer_array(f, kArrBo, 0, true, (double *)st[f].old_cell_magnetic))
-      return -1;
-    for (int d = 0; d < 3; ++d)
-      if (transfer_array(f, kArrP, d, true, st[f].face_flux[d]) ||
-          transfer_array(f, kArrPo, d, true, st[f].old_face_flux[d]))
-        return -1;
-  }
-  return 0;
+  return move_state(st, true);
 }
 
 int Context::download_state(gamera_no_storage st[kFaces], int scratch) {
+  if (move_state(st, false) != 0) return -1;
   for (int f = 0; f < kFaces; ++f) {
-    if (transfer_array(f, kArrU, 0, false, st[f].conserved) ||
-        transfer_array(f, kArrUo, 0, false, st[f].old_conserved) ||
-        transfer_array(f, kArrB, 0, false, (double *)st[f].cell_magnetic) ||
-        transfer_array(f, kArrBo, 0, false, (double *)st[f].old_cell_magnetic))
-      return -1;
-    for (int d = 0; d < 3; ++d)
-      if (transfer_array(f, kArrP, d, false, st[f].face_flux[d]) ||
-          transfer_array(f, kArrPo, d, false, st[f].old_face_flux[d]))
-        return -1;
     if (scratch) {
       if (transfer_array(f, kArrUp, 0, false, st[f].predicted_conserved) ||
           transfer_array(f, kArrBp, 0, false,
