@@ -69,7 +69,7 @@ struct System {
   int max_iter;
   int pad;
   const int *gate;  // when set, the solve runs only where *gate != 0
-  // Variable Pedersen conductance (Hall = 0) when coef is set (k_pcg only):
+  // Variable Pedersen conductance (Hall = 0) when coef is set:
   // the five-point stencil of the conductance-tensor operator
   // (nonorthogonal_mi.c:776-865) per reduced unknown -- diagonal, lower,
   // upper, longitude lower, longitude upper, `unknowns` entries each -- the
@@ -452,16 +452,46 @@ __global__ void __launch_bounds__(kThreads, 1)
 
 // ------------------------------------------------------- column kernel
 // The same solve with one thread per longitude column of the band: thread
-// j keeps the band's column of s, x, r and A s in registers (MR rows at
-// most), takes the vertical stencil neighbours from its own registers and
-// only the longitude neighbours from shared memory.  Used when the grid fits
-// (np <= col_threads(MR), band rows <= MR); k_pcg serves the rest.
+// j keeps the band's column of x, r, p, s = A p and w = A z in registers (MR
+// rows at most), takes the vertical stencil neighbours from its own column
+// and only the longitude neighbours from shared memory.  Used when the grid
+// fits (np <= col_threads(MR), band rows <= MR); k_pcg serves the rest.
+//
+// The iteration is the conjugate gradient method with its two dot products
+// moved together (Chronopoulos and Gear, J. Comput. Appl. Math. 25, 1989):
+// with z = M^-1 r and w = A z, gamma = r.z and delta = w.z,
+//   beta = gamma / gamma_old, alpha = gamma / (delta - beta gamma / alpha_old),
+//   p = z + beta p, s = w + beta s, x += alpha p, r -= alpha s,
+// the iterates of the usual form up to rounding with one reduction over the
+// cluster per iteration.  The bound is latency: a push and a cluster barrier
+// cost about 0.7 us, and the two of the usual form were the larger part of an
+// iteration.  The neighbours' edge rows of z that A z needs are advanced by
+// each CTA itself (the recurrences of s, r and z on copies of those rows),
+// so all that crosses between CTAs is the edge rows of w, pushed with the
+// partial sums.
+//
+// kVar: variable Pedersen conductance, Hall = 0; the edge coefficients of the
+// band (vertical and longitude edges, shared by the two points beside them)
+// and the reciprocal diagonal are kept in shared memory.
+//
+// Measured (both hemispheres in a launch): 361 x 181 variable Pedersen 12.2 ->
+// 5.8 us an iteration (its coefficients came from L2, the points were walked
+// by 512 threads); constant Pedersen 5.4 -> 5.1; 192 x 22 2.7 -> 2.4.
 
 __host__ __device__ constexpr int col_threads(int mr) {
   return mr <= 4 ? 512 : (mr <= 12 ? 384 : 256);
 }
 
-template <int MR>
+// With 12 rows at 384 threads (168 registers) x, touched once an iteration,
+// lives in shared memory: the five vectors in registers spill.
+__host__ __device__ constexpr bool col_x_shared(int mr) { return mr == 12; }
+
+// Row constants of the reduced system with the row weight folded in.
+struct __align__(16) ColRow {
+  double lo, up, lon, rdg, rw, pad;
+};
+
+template <int MR, bool kVar>
 __global__ void __launch_bounds__(col_threads(MR), 1)
     k_pcg_col(const System *systems, int csize) {
   cg::cluster_group cl = cg::this_cluster();
@@ -469,103 +499,160 @@ __global__ void __launch_bounds__(col_threads(MR), 1)
   const System &S = systems[blockIdx.x / csize];
   if (S.gate != nullptr && *S.gate == 0) return;
   const int np = S.np, R = S.nt - 2;
-  const int j = threadIdx.x;
-  const bool on = j < np;
+  const bool on = (int)threadIdx.x < np;
+  // threads past the last longitude repeat it; their sums and stores are
+  // dropped
+  const int j = on ? (int)threadIdx.x : np - 1;
   const int jm = j == 0 ? np - 1 : j - 1;
-  const int jp = j + 1 >= np ? 0 : j + 1;
+  const int jp = j + 1 == np ? 0 : j + 1;
 
   extern __shared__ __align__(16) double dyn[];
   __shared__ double wbuf[32 * kSlotWidth];
   __shared__ double slots[kSlots * kMaxCluster * kSlotWidth];
-  __shared__ double pole_s;
 
-  // halo rows: [0] s above, [np] z above, [2np] s below, [3np] z below
   const int ra = (int)((long long)rank * R / csize);
   const int nrow = (int)((long long)(rank + 1) * R / csize) - ra;
   const bool top = rank == 0, bottom = rank == csize - 1;
-  double *ssm = dyn;                    // MR rows of s
-  double *halo = dyn + (size_t)MR * np;
-  Row *rt = reinterpret_cast<Row *>(halo + 4 * (size_t)np);
-  // the neighbours' halo rows that this band's edge rows feed
-  double *peer_up = top ? nullptr : cl.map_shared_rank(halo, rank - 1) + 2 * np + j;
-  double *peer_dn = bottom ? nullptr : cl.map_shared_rank(halo, rank + 1) + j;
-  for (int l = j; l < nrow; l += blockDim.x) rt[l] = S.rows[ra + l];
+  // MR + 1 rows of the vector A is applied to: the band's, then the next
+  // band's first row (0 below the last band), then zeros
+  ColRow *rt = reinterpret_cast<ColRow *>(dyn);   // 16-byte aligned, unlike odd rows of np
+  double *zs = dyn + MR * (sizeof(ColRow) / sizeof(double));
+  double *edge = zs + (size_t)(MR + 1) * np;   // [parity][0 above, 1 below][np]
+  double *vert = edge + 4 * (size_t)np;  // kVar: [MR + 1][np] edge to the row below
+  double *lon = vert + (kVar ? (size_t)(MR + 1) * np : 0);  // [MR][np] edge to j - 1
+  double *rdiag = lon + (kVar ? (size_t)MR * np : 0);       // [MR][np]
+  double *xs = rdiag + (kVar ? (size_t)MR * np : 0);        // [MR][np] x, where not in registers
+  // where this band's first and last row go in the neighbours' edge rows
+  double *peer_up = top ? nullptr : cl.map_shared_rank(edge, rank - 1) + np + j;
+  double *peer_dn = bottom ? nullptr : cl.map_shared_rank(edge, rank + 1) + j;
+  // rows past the band's have zero coefficients, so the loops over MR rows
+  // have no branch and the rows' chains of operations overlap
+  for (int l = threadIdx.x; l < MR; l += blockDim.x) {
+    const Row rw = S.rows[ra + (l < nrow ? l : 0)];
+    rt[l] = l < nrow ? ColRow{rw.w * rw.lo, rw.w * rw.up, rw.w * rw.lon, rw.rdg, rw.rw, 0.0}
+                     : ColRow{0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  }
+  for (int q = threadIdx.x; q < (MR + 1) * np; q += blockDim.x) zs[q] = 0.0;
+  // reciprocal diagonal of the rows beside the band
+  double rdg_up = 0.0, rdg_dn = 0.0;
+  if (kVar) {
+    const long long n = S.unknowns;
+    for (int q = threadIdx.x; q < (MR + 1) * np; q += blockDim.x) {
+      const bool in = q < nrow * np, past = !in && q < (nrow + 1) * np;
+      const long long ci = 1 + (long long)ra * np + q;
+      vert[q] = in ? -S.coef[n + ci] : past ? -S.coef[2 * n + ci - np] : 0.0;
+      if (q < MR * np) {
+        lon[q] = in ? -S.coef[3 * n + ci] : 0.0;
+        rdiag[q] = in ? 1.0 / S.coef[ci] : 0.0;
+      }
+    }
+    if (!top) rdg_up = 1.0 / S.coef[1 + (long long)(ra - 1) * np + j];
+    if (!bottom) rdg_dn = 1.0 / S.coef[1 + (long long)(ra + nrow) * np + j];
+  } else {
+    if (!top) rdg_up = S.rows[ra - 1].rdg;
+    if (!bottom) rdg_dn = S.rows[ra + nrow].rdg;
+  }
   const bool lead = top;
   const double dnp = (double)np;
-  const double ps = dnp * S.pe;
-  int ctr = 0;
+  const double pe = S.pe, diag0 = S.diag0;
+  const double ps = dnp * pe;           // pole residual scale
+  const double pd = kVar ? diag0 : ps;  // pole diagonal
+  const double pedge = kVar ? S.pedge[j] : 1.0;
+  int ctr = 0, par = 0;
 
-  double sv[MR], xv[MR], rv[MR], av[MR];
-
-  // s of row l := v, in registers, shared memory and the neighbours' halos
-  auto put_s = [&](int l, double v) {
-    sv[l] = v;
-    ssm[l * np + j] = v;
-    if (l == 0 && !top) peer_up[0] = v;
-    if (l == nrow - 1 && !bottom) peer_dn[0] = v;
+  constexpr bool kXs = col_x_shared(MR);
+  double xreg[kXs ? 1 : MR], rv[MR], pv[MR], sv[MR], wv[MR];
+  auto get_x = [&](int l) { return kXs ? xs[l * np + j] : xreg[kXs ? 0 : l]; };
+  auto put_x = [&](int l, double v) {
+    if (!kXs)
+      xreg[kXs ? 0 : l] = v;
+    else if (on)
+      xs[l * np + j] = v;
   };
-  // A s of row l from the registers of the column (nonorthogonal_mi.c:394-409)
-  auto stencil = [&](int l, const Row &rw, double pole) {
-    const double c = sv[l];
-    const double sm = ssm[l * np + jm];
-    const double sp = ssm[l * np + jp];
-    const double lv = l > 0 ? sv[l > 0 ? l - 1 : 0] : (top ? pole : halo[j]);
-    const double uv = l < nrow - 1 ? sv[l + 1 < MR ? l + 1 : MR - 1]
-                                   : (bottom ? 0.0 : halo[2 * np + j]);
-    return rw.w * (rw.lo * (c - lv) + rw.up * (c - uv) +
-                   rw.lon * (2.0 * c - sm - sp));
-  };
+  double r_up = 0.0, s_up = 0.0, z_up = 0.0, r_dn = 0.0, s_dn = 0.0, z_dn = 0.0;
+  double x0 = 0.0, r0 = 0.0, p0 = 0.0, s0 = 0.0, z0 = 0.0, w0 = 0.0;
 
-  double x0 = 0.0, r0 = 0.0;
+  auto rdg_of = [&](int l) { return kVar ? rdiag[l * np + j] : rt[l].rdg; };
+  // first and last row of v to the neighbours' edge rows of the next parity
+  auto push_row = [&](int l, double v) {
+    if (!on) return;
+    const int at = (par ^ 1) * 2 * np;
+    if (l == 0 && !top) peer_up[at] = v;
+    if (l == nrow - 1 && !bottom) peer_dn[at] = v;
+  };
+  // A v of row l (nonorthogonal_mi.c:394-409, :872-897 with Hall = 0), v in zs;
+  // below and above are the column's neighbouring values
+  auto stencil = [&](int l, double c, double below, double above) {
+    const double west = zs[l * np + jm], east = zs[l * np + jp];
+    if (kVar) {
+      double a = vert[l * np + j] * (c - below);
+      a = fma(vert[(l + 1) * np + j], c - above, a);
+      a = fma(lon[l * np + j], c - west, a);
+      return fma(lon[l * np + jp], c - east, a);
+    }
+    const ColRow rw = rt[l];
+    double a = rw.lo * (c - below);
+    a = fma(rw.up, c - above, a);
+    return fma(rw.lon, (c - west) + (c - east), a);
+  };
+  // pole row of A v from the ring sum of v (kVar: weighted by the pole edges)
+  auto pole_row = [&](double v0, double ring) {
+    return kVar ? diag0 * v0 - ring : pe * (dnp * v0 - ring);
+  };
+  auto ring_term = [&](double v) { return kVar ? pedge * v : v; };
+
+#pragma unroll
+  for (int l = 0; l < MR; ++l) {
+    rv[l] = pv[l] = sv[l] = wv[l] = 0.0;
+    const double v = l < nrow ? S.pot[(size_t)(ra + l + 1) * np + j] : 0.0;
+    put_x(l, isfinite(v) ? v : 0.0);
+  }
   if (lead) {
     double pm[1] = {0.0};
-    for (int q = j; q < np; q += blockDim.x) {
-      const double v = S.pot[q];
-      if (isfinite(v)) pm[0] += v / dnp;
-    }
+    const double v = S.pot[j];
+    if (on && isfinite(v)) pm[0] = v / dnp;
     block_sum<1>(pm, wbuf);
     x0 = pm[0];
   }
-#pragma unroll
-  for (int l = 0; l < MR; ++l) {
-    xv[l] = 0.0;
-    rv[l] = 0.0;
-    av[l] = 0.0;
-    sv[l] = 0.0;
-    if (l < nrow && on) {
-      const double v = S.pot[(size_t)(ra + l + 1) * np + j];
-      xv[l] = isfinite(v) ? v : 0.0;
-      put_s(l, xv[l]);
-    }
-  }
-  if (lead && j == 0) pole_s = x0;
   cl.sync();
 
+  // r = rhs - A x, {norm^2, rhs^2, non-finite FAC} over the cluster
   auto true_residual = [&](double (&out)[3]) {
-    double v[4] = {0.0, 0.0, 0.0, 0.0};  // norm^2, rhs^2, bad, ring
-    const double pole = lead ? pole_s : 0.0;
 #pragma unroll
     for (int l = 0; l < MR; ++l) {
-      if (l < nrow && on) {
-        const Row rw = rt[l];
+      const double x = get_x(l);
+      if (on && l < nrow) zs[l * np + j] = x;
+      push_row(l, x);
+    }
+    cl.sync();
+    par ^= 1;
+    const double x_up = top ? x0 : edge[par * 2 * np + j];
+    if (on && !bottom) zs[nrow * np + j] = edge[par * 2 * np + np + j];
+    double v[4] = {0.0, 0.0, 0.0, 0.0};  // norm^2, rhs^2, bad, ring
+#pragma unroll
+    for (int l = 0; l < MR; ++l) {
+      if (l < nrow) {
+        const Row rw = S.rows[ra + l];
         const double f = S.fac[(size_t)(ra + l + 1) * np + j];
         const double u = S.neg_r2 * f * rw.inc;
-        const double rhs = rw.w * u + rw.extra;
-        rv[l] = rhs - stencil(l, rw, pole);
+        const double rhs = rw.w * u + (kVar ? 0.0 : rw.extra);
+        const double x = zs[l * np + j];
+        rv[l] = rhs - stencil(l, x, l > 0 ? zs[(l - 1) * np + j] : x_up,
+                              zs[(l + 1) * np + j]);
         const double q = rv[l] * rw.rw;
         v[0] += q * q;
         v[1] += u * u;
         v[2] += isfinite(f) ? 0.0 : 1.0;
-        if (l == 0 && top) v[3] += sv[0];
+        if (l == 0 && top) v[3] = ring_term(x);
       }
     }
+    if (!on) v[0] = v[1] = v[2] = v[3] = 0.0;
     block_sum<4>(v, wbuf);
     if (lead) {
-      const double ax0 = S.pe * (dnp * pole - v[3]);
-      r0 = 0.0 - ax0;
+      r0 = 0.0 - pole_row(x0, v[3]);
       const double pr = r0 / ps;
       v[0] += dnp * pr * pr;
-      v[1] += dnp * S.low * S.low;
+      if (!kVar) v[1] += dnp * S.low * S.low;
     }
     out[0] = v[0];
     out[1] = v[1];
@@ -573,24 +660,64 @@ __global__ void __launch_bounds__(col_threads(MR), 1)
     cluster_sum<3>(cl, out, slots, ctr, rank, csize);
   };
 
-  auto restart = [&]() -> double {
-    double v[1] = {0.0};
+  // w = A z with z in zs and z_up, z_dn, z0 current; adds w.z and the ring
+  // sum of z to v[2], v[3], then sums {norm^2, r.z, w.z} over the cluster
+  // into out, the edge rows of w crossing with the sums
+  auto apply_and_sum = [&](double (&v)[4], double (&out)[3]) {
+    // the column walked once: each of its values is read once, one row ahead
+    double below = top ? z0 : z_up, c = zs[j];
+    if (top) v[3] = ring_term(c);
 #pragma unroll
     for (int l = 0; l < MR; ++l) {
-      if (l < nrow && on) {
-        const double z = rv[l] * rt[l].rdg;
-        put_s(l, z);
-        v[0] += rv[l] * z;
-      }
+      const double above = zs[(l + 1) * np + j];
+      const double a = stencil(l, c, below, above);
+      // kVar: the row past the band has the edge above it
+      wv[l] = kVar && l >= nrow ? 0.0 : a;
+      v[2] = fma(wv[l], c, v[2]);
+      below = c;
+      c = above;
     }
-    block_sum<1>(v, wbuf);
+#pragma unroll
+    for (int l = 0; l < MR; ++l) push_row(l, wv[l]);
+    if (!on) v[0] = v[1] = v[2] = v[3] = 0.0;
+    block_sum<4>(v, wbuf);
     if (lead) {
-      const double z0 = r0 / ps;
-      v[0] += r0 * z0;
-      if (j == 0) pole_s = z0;
+      w0 = pole_row(z0, v[3]);
+      const double pr = r0 / ps;
+      v[0] = fma(dnp * pr, pr, v[0]);
+      v[1] = fma(r0, z0, v[1]);
+      v[2] = fma(z0, w0, v[2]);
     }
-    cluster_sum<1>(cl, v, slots, ctr, rank, csize);
-    return v[0];
+    out[0] = v[0];
+    out[1] = v[1];
+    out[2] = v[2];
+    cluster_sum<3>(cl, out, slots, ctr, rank, csize);
+    par ^= 1;
+  };
+
+  // z = M^-1 r and w = A z from the true residual, p = s = 0
+  auto restart = [&](double (&out)[3]) {
+#pragma unroll
+    for (int l = 0; l < MR; ++l) push_row(l, rv[l]);
+    cl.sync();
+    par ^= 1;
+    r_up = top ? 0.0 : edge[par * 2 * np + j];
+    r_dn = bottom ? 0.0 : edge[par * 2 * np + np + j];
+    z_up = r_up * rdg_up;
+    z_dn = r_dn * rdg_dn;
+    s_up = s_dn = p0 = s0 = 0.0;
+    z0 = r0 / pd;
+    double v[4] = {0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+    for (int l = 0; l < MR; ++l) {
+      const double z = rv[l] * rdg_of(l);
+      if (on && l < nrow) zs[l * np + j] = z;
+      v[1] = fma(rv[l], z, v[1]);
+      pv[l] = sv[l] = 0.0;
+    }
+    if (on && !bottom) zs[nrow * np + j] = z_dn;
+    __syncthreads();
+    apply_and_sum(v, out);
   };
 
   double tr[3];
@@ -605,103 +732,82 @@ __global__ void __launch_bounds__(col_threads(MR), 1)
   const int max_iter = S.max_iter < kMaxIterations ? S.max_iter : kMaxIterations;
 
   if (!bad && !conv) {
-    double rho = restart();
+    double sums[3];
+    restart(sums);
+    double gamma = sums[1], den = sums[2], beta = 0.0;
     for (int it = 1; it <= max_iter; ++it) {
-      if (!isfinite(rho) || rho <= DBL_MIN) break;
-      double v[2] = {0.0, 0.0};  // s.As, first-ring sum of s
-      const double pole = lead ? pole_s : 0.0;
+      if (!isfinite(gamma) || gamma <= DBL_MIN) break;
+      if (!isfinite(den) || den <= DBL_MIN) break;
+      const double alpha = gamma / den;
+      // copies of the neighbours' edge rows
+      if (!top) {
+        s_up = fma(beta, s_up, edge[par * 2 * np + j]);
+        r_up = fma(-alpha, s_up, r_up);
+        z_up = r_up * rdg_up;
+      }
+      if (!bottom) {
+        s_dn = fma(beta, s_dn, edge[par * 2 * np + np + j]);
+        r_dn = fma(-alpha, s_dn, r_dn);
+        z_dn = r_dn * rdg_dn;
+      }
+      if (lead) {
+        p0 = fma(beta, p0, z0);
+        s0 = fma(beta, s0, w0);
+        x0 = fma(alpha, p0, x0);
+        r0 = fma(-alpha, s0, r0);
+        z0 = r0 / pd;
+      }
+      double v[4] = {0.0, 0.0, 0.0, 0.0};  // norm^2, r.z, w.z, ring
 #pragma unroll
       for (int l = 0; l < MR; ++l) {
-        if (l < nrow && on) {
-          av[l] = stencil(l, rt[l], pole);
-          v[0] += sv[l] * av[l];
-          if (l == 0 && top) v[1] += sv[0];
-        }
+        const double rdg = rdg_of(l);
+        pv[l] = fma(beta, pv[l], rv[l] * rdg);
+        sv[l] = fma(beta, sv[l], wv[l]);
+        put_x(l, fma(alpha, pv[l], get_x(l)));
+        rv[l] = fma(-alpha, sv[l], rv[l]);
+        const double z = rv[l] * rdg, q = rv[l] * rt[l].rw;
+        if (on && l < nrow) zs[l * np + j] = z;
+        v[0] = fma(q, q, v[0]);
+        v[1] = fma(rv[l], z, v[1]);
       }
-      block_sum<2>(v, wbuf);
-      double As0 = 0.0;
-      double den[1] = {v[0]};
-      if (lead) {
-        As0 = S.pe * (dnp * pole - v[1]);
-        den[0] += pole * As0;
-      }
-      cluster_sum<1>(cl, den, slots, ctr, rank, csize);
-      if (!isfinite(den[0]) || den[0] <= DBL_MIN) break;
-      const double alpha = rho / den[0];
-      double w2[2] = {0.0, 0.0};
-#pragma unroll
-      for (int l = 0; l < MR; ++l) {
-        if (l < nrow && on) {
-          const Row &rw = rt[l];
-          xv[l] += alpha * sv[l];
-          rv[l] -= alpha * av[l];
-          const double q = rv[l] * rw.rw;
-          const double z = rv[l] * rw.rdg;
-          w2[0] += q * q;
-          w2[1] += rv[l] * z;
-          if (l == 0 && !top) peer_up[np] = z;
-          if (l == nrow - 1 && !bottom) peer_dn[np] = z;
-        }
-      }
-      block_sum<2>(w2, wbuf);
-      if (lead) {
-        x0 += alpha * pole;
-        r0 -= alpha * As0;
-        const double pr = r0 / ps;
-        w2[0] += dnp * pr * pr;
-        w2[1] += r0 * (r0 / ps);
-      }
-      cluster_sum<2>(cl, w2, slots, ctr, rank, csize);
-      final_res = sqrt(fmax(0.0, w2[0]));
+      if (on && !bottom) zs[nrow * np + j] = z_dn;
+      __syncthreads();
+      apply_and_sum(v, sums);
+      final_res = sqrt(fmax(0.0, sums[0]));
       iters = it;
       if (final_res <= target || it % kTruePeriod == 0) {
-#pragma unroll
-        for (int l = 0; l < MR; ++l)
-          if (l < nrow && on) put_s(l, xv[l]);
-        if (lead && j == 0) pole_s = x0;
-        cl.sync();
+        // verified with the true residual (nonorthogonal_mi.c:562-582)
         true_residual(tr);
         final_res = sqrt(fmax(0.0, tr[0]));
         if (final_res <= target) {
           conv = 1;
           break;
         }
-        rho = restart();
+        restart(sums);
+        gamma = sums[1];
+        den = sums[2];
+        beta = 0.0;
         continue;
       }
-      const double rho_new = w2[1];
-      if (!isfinite(rho_new) || rho_new <= DBL_MIN) break;
-      const double beta = rho_new / rho;
-#pragma unroll
-      for (int l = 0; l < MR; ++l) {
-        if (l < nrow && on) {
-          sv[l] = rv[l] * rt[l].rdg + beta * sv[l];
-          ssm[l * np + j] = sv[l];
-        }
-      }
-      if (on) {
-        if (!top) halo[j] = halo[np + j] + beta * halo[j];
-        if (!bottom) halo[2 * np + j] = halo[3 * np + j] + beta * halo[2 * np + j];
-      }
-      if (lead && j == 0) pole_s = r0 / ps + beta * pole;
-      rho = rho_new;
-      __syncthreads();
+      beta = sums[1] / gamma;
+      gamma = sums[1];
+      den = sums[2] - beta * gamma / alpha;
     }
   }
 
   if (bad) {
-    if (lead && j == 0) *S.status = 2;
+    if (lead && threadIdx.x == 0) *S.status = 2;
     cl.sync();  // no CTA leaves while a peer may still write its memory
     return;
   }
 #pragma unroll
   for (int l = 0; l < MR; ++l)
-    if (l < nrow && on) S.pot[(size_t)(ra + l + 1) * np + j] = xv[l];
-  if (lead)
-    for (int q = j; q < np; q += blockDim.x) S.pot[q] = x0;
-  if (bottom)
-    for (int q = j; q < np; q += blockDim.x) S.pot[(size_t)(S.nt - 1) * np + q] = S.low;
-  if (lead && j == 0) {
+    if (l < nrow && on) S.pot[(size_t)(ra + l + 1) * np + j] = get_x(l);
+  if (on) {
+    if (lead) S.pot[j] = x0;
+    if (bottom) S.pot[(size_t)(S.nt - 1) * np + j] = S.low;
+  }
+  if (lead && threadIdx.x == 0) {
     *S.stats = gamera_mi_solver_stats{iters, initial, final_res, conv};
     *S.status = conv ? 0 : 1;
   }
@@ -947,17 +1053,20 @@ bool launchable(const Shape &sh) {
   return n >= 1;
 }
 
-// Column kernel: MR rows of s plus four halo rows, and the row table.
-size_t col_smem(int mr, int np) {
-  return ((size_t)mr * np + 4 * (size_t)np) * sizeof(double) + (size_t)mr * sizeof(Row);
+// Column kernel: MR + 1 rows of z, four edge rows, with variable conductance the
+// band's edge coefficients and reciprocal diagonal, and the row table.
+size_t col_smem(int mr, int np, bool variable) {
+  const size_t rows = (size_t)mr + 5 + (variable ? 3 * (size_t)mr + 1 : 0) +
+                      (col_x_shared(mr) ? (size_t)mr : 0);
+  return rows * np * sizeof(double) + (size_t)mr * sizeof(ColRow);
 }
 
-PcgKernel col_kernel(int mr) {
+PcgKernel col_kernel(int mr, bool variable) {
   switch (mr) {
-    case 4: return k_pcg_col<4>;
-    case 8: return k_pcg_col<8>;
-    case 12: return k_pcg_col<12>;
-    case 16: return k_pcg_col<16>;
+    case 4: return variable ? k_pcg_col<4, true> : k_pcg_col<4, false>;
+    case 8: return variable ? k_pcg_col<8, true> : k_pcg_col<8, false>;
+    case 12: return variable ? k_pcg_col<12, true> : k_pcg_col<12, false>;
+    case 16: return variable ? k_pcg_col<16, true> : k_pcg_col<16, false>;
     default: return nullptr;
   }
 }
@@ -1016,24 +1125,22 @@ bool cuda_ok(cudaError_t e, const char *what) {
   return false;
 }
 
-// Cluster size: about 2048 unknowns per CTA, at most 16 CTAs (8 where the
-// device cannot co-schedule 16), every CTA owning at least one row.
 // Launch shape: the column kernel with the smallest band (most CTAs, at
-// most 16) whose rows fit its registers; otherwise the shared-memory kernel
+// most 16) whose rows fit its registers: an iteration costs a barrier whatever
+// the cluster and each row adds to it (192 x 22: bands of 4 rows 0.93 ms, 8
+// rows 1.10, 12 rows 1.72); otherwise the shared-memory kernel
 // with about 2048 unknowns per CTA (8 CTAs at most where the device cannot
 // co-schedule 16).
-int choose_shape(gcs_mi_plan *p, bool variable = false) {
+int choose_shape(gcs_mi_plan *p, bool variable) {
   const int R = p->nt - 2, np = p->np;
   const int threads = (np + 31) / 32 * 32;
-  // the variable-conductance mode lives in the shared-memory kernel
   for (int mr : {4, 8, 12, 16}) {
-    if (variable) break;
     Shape sh;
-    sh.kernel = col_kernel(mr);
+    sh.kernel = col_kernel(mr, variable);
     sh.csize = (R + mr - 1) / mr;
     sh.threads = threads;
     sh.rows = mr;
-    sh.smem = col_smem(mr, np);
+    sh.smem = col_smem(mr, np, variable);
     if (threads > col_threads(mr) || sh.csize > kMaxCluster) continue;
     if (launchable(sh)) {
       p->shape = sh;
