@@ -5,22 +5,31 @@
 // cluster that keeps every vector in L2.
 //
 // Layout.  The interior unknowns (rows r = 0..R-1 for colatitude rows
-// 1..nt-2, longitudes j = 0..np-1) are stored skewed by anti-diagonal: the
-// points with r + j = d form one column of Rp doubles (Rp = 32 M >= R rows),
-// column F + d, row r at position (r mod M) 32 + r / M of the column.  The
-// pole unknown sits at index 0.  Padding rows, off-grid positions of a
-// diagonal and the F padding columns hold zeros and stay zero through every
+// 1..nt-2, longitudes j = 0..np-1) are stored in blocks of 64 rows, one block
+// per sweep warp, skewed inside the block: lane l of the warp holds rows 2l
+// and 2l + 1, and the points with l + j = d form column kPad + d of the
+// block, 64 doubles with row r of the block at position r.  The pole unknown
+// sits at index 0.  Padding rows, off-grid positions of a column and the
+// padding columns on both sides hold zeros and stay zero through every
 // operation.
 //
 // SSOR.  The lexicographic forward sweep and the reverse sweep are
-// wavefronts along anti-diagonals: point (r, j) depends on (r-1, j),
-// (r, j-1) and on the periodic seam (r, 0).  One warp runs a sweep, lane l
-// holding rows l M .. l M + M - 1 as M independent chains, so one step
-// advances the whole anti-diagonal.  Whole diagonals move between global
-// and shared memory by bulk asynchronous copies (tracked by mbarriers,
-// every wait bounded), several diagonals per copy.  The preconditioner is
-// the reference's (D + L) D^-1 (D + U) with the triangular solves done on
-// D^-1-scaled rows, so it equals the reference's to rounding.
+// wavefronts: point (r, j) depends on (r-1, j), (r, j-1) and on the periodic
+// seam (r, 0).  One step of a sweep warp advances one column: lane l computes
+// its two rows at longitude t - l, the first from the neighbour lane's second
+// row of the previous step (one warp shuffle), the second from the first.  A
+// block therefore takes np + 31 steps, and the warps of successive blocks,
+// on different CTAs, follow one another by some forty steps; the row between
+// two blocks crosses through distributed shared memory.  Values and
+// coefficients are prefetched from L2 into a shared-memory ring by cp.async,
+// each lane copying what it will read itself, so the sweep needs no barrier
+// inside a warp beyond the shuffle.  The preconditioner is the reference's
+// (D + L) D^-1 (D + U) with the triangular solves done on D^-1-scaled rows,
+// so it equals the reference's to rounding.
+//
+// Bound: the chain of a step (a shuffle and two dependent fused
+// multiply-adds).  Two rows per lane make np + R / 2 steps of the chain where
+// one row per lane would make np + R with a chain one multiply-add shorter.
 //
 // Band schedule (the default on grids narrower than 17 longitudes): the
 // same sweeps with the rows split into one band per CTA, each band swept by
@@ -30,7 +39,7 @@
 //
 // Vector updates, stencil applications and dot products run on all CTAs
 // of the cluster (dot products summed in a fixed order, identical on every
-// CTA); the sweeps run on one warp of CTA 0 between two cluster barriers.
+// CTA), between cluster barriers.
 // The BiCGStab iterates therefore differ from the CPU solver's at rounding
 // level, and a converged solve meets the same residual target.
 #include <cooperative_groups.h>
@@ -53,19 +62,16 @@ using gcs::set_api_error;
 
 namespace {
 
-// The sweep warp holds 32 M interior colatitude rows (rows padded to
-// Rp = 32 M): M = 1..8 (up to 256 rows) or 16 (up to 512 rows).  It moves
-// diagonals in groups of 12 (a 36-diagonal prefetch ring) where the seam
-// allows (at least 25 longitudes) and shared memory fits (up to 6 chains),
-// else in groups of 8 (24 diagonals; at least 17 longitudes), of 4 (16
-// diagonals; 8 for M = 16), or of 1 for grids of fewer than 9 longitudes:
-// every group pays a fixed synchronisation cost in the sweep warp, so
-// larger groups are faster.
+// Sweep blocks of 64 rows (two per lane), up to 8 of them.  A sweep warp
+// works in groups of kGroup steps and prefetches its operands up to 24 steps
+// ahead into a ring of kRing: an L2 round trip of some 700 cycles is about 12
+// steps.
+constexpr int kRing = 32;
 constexpr int kThreads = 256;
 constexpr int kMaxRows = 512;
-constexpr int kPad = 16;                    // padding diagonals on each side (>= group - 1)
-constexpr unsigned kSpinLimit = 1u << 20;   // polls of a sweep copy's mbarrier
-constexpr unsigned kDrainLimit = 1u << 16;  // polls per copy after an abort
+constexpr int kBlockRows = 64;
+constexpr int kGroup = 8;
+constexpr int kPad = 16;                    // padding columns on each side (>= group - 1)
 constexpr int kMaxCluster = 16;
 constexpr int kSlots = 4;
 constexpr int kSlotWidth = 4;
@@ -73,6 +79,7 @@ constexpr int kRestart = 256;
 constexpr int kMaxIterations = 1 << 20;
 constexpr int kMaxLongitudes = 8192;        // pole-edge table in shared memory
 constexpr size_t kSmemCap = 220 * 1024;     // dynamic shared memory of a launch
+constexpr size_t kStepBytes = 48 * 32;      // ring bytes of a step: 2 values, 2 coefficient pairs a lane
 
 // Per-row constants of the full polar grid, computed on the host with the
 // reference's formulas (nonorthogonal_mi.c:643-656, :776-865).
@@ -84,16 +91,21 @@ struct TRow {
 };
 
 struct TSys {
-  int np, nt, R, Rp, max_iter;
-  unsigned core0, core1;  // skewed index range of the grid's diagonals
+  int np, nt, R, max_iter;
+  int blocks;             // sweep blocks of 64 rows
+  int cols;               // columns of a block
+  unsigned core0, core1;  // index range of the unknowns, padding between blocks included
   double dth, dph, neg_r2, pole_sin, pole_inc2, ps, abs_tol, rel_tol;
-  const TRow *rows;             // max(nt, Rp + 2) rows; padding rows have s = 1
+  const TRow *rows;             // nt rows
+  unsigned *loc;                // (row + 1) << 13 | longitude of each index, 0 off the grid
   const double *fac, *sp, *sh;  // natural layout (nt x np)
   double *pot;                  // natural layout, initial guess in, solution out
   // skewed vectors
   double *rhs, *x, *res, *shd, *srch, *as, *psv, *mid, *pm, *am, *fw, *pin;
+  double *wt;   // 1 / sin(theta) of the row: weight of the residual norm, 0 off the grid
   // skewed stencil: raw coefficients and the D^-1-scaled sweep pairs
   double *dg, *lo, *up, *ll, *lu, *rdg;
+  // (coefficient position of row r in its column: 32 (r mod 2) + lane)
   double2 *cf;  // (lo, ll) / dg: forward sweep
   double2 *cb;  // (up, lu) / dg: reverse sweep
   double *pe;   // pole edge coefficients (np)
@@ -106,20 +118,22 @@ struct TSys {
   int nbands;   // bands (CTAs 0 .. nbands - 1 sweep)
 };
 
-// Position of row r inside a diagonal of Rp = 32 M rows: the sweep warp's
-// lane r / M holds it as chain r % M, at position (r % M) 32 + r / M.
-__device__ __forceinline__ int row_pos(int Rp, int r) {
-  const int M = Rp >> 5;
-  return (r % M) * 32 + r / M;
+// Index of row r, longitude j in the vectors, and in the coefficient pairs.
+__device__ __forceinline__ size_t col_of(int cols, int r, int j) {
+  return (size_t)(r >> 6) * cols + kPad + ((r & 63) >> 1) + j;
 }
-__device__ __forceinline__ int pos_row(int Rp, int q) {
-  const int M = Rp >> 5;
-  return (q & 31) * M + (q >> 5);
+__device__ __forceinline__ size_t sidx(int cols, int r, int j) {
+  return col_of(cols, r, j) * kBlockRows + (r & 63);
 }
-
-// Skewed index of row r, longitude j.
-__device__ __forceinline__ size_t sidx(int Rp, int r, int j) {
-  return (size_t)(kPad + r + j) * Rp + row_pos(Rp, r);
+__device__ __forceinline__ size_t cidx(int cols, int r, int j) {
+  return col_of(cols, r, j) * kBlockRows + 32 * (r & 1) + ((r & 63) >> 1);
+}
+// Index of the row below (r - 1) and above (r + 1) at the same longitude j.
+__device__ __forceinline__ size_t below(int cols, size_t k, int r, int j) {
+  return (r & 63) == 0 ? sidx(cols, r - 1, j) : k - 1 - ((r & 1) ? 0 : kBlockRows);
+}
+__device__ __forceinline__ size_t above(int cols, size_t k, int r, int j) {
+  return (r & 63) == 63 ? sidx(cols, r + 1, j) : k + 1 + ((r & 1) ? kBlockRows : 0);
 }
 
 __device__ __forceinline__ double warp_sum(double v) {
@@ -167,234 +181,6 @@ struct Reducer {
 
 __device__ __forceinline__ unsigned smem_u32(const void *p) {
   return (unsigned)__cvta_generic_to_shared(p);
-}
-
-// Shared memory of the sweep warp.  Ring: kRG slots of G anti-diagonals
-// (G Rp values and G Rp coefficient pairs each) filled by two bulk
-// asynchronous copies per group, one mbarrier per slot; group n of the
-// warp's running group count uses slot n mod kRG and completes phase
-// n / kRG of its barrier.  Stage: two halves of G output diagonals,
-// drained to global memory by one bulk copy per group.  edge: each row's
-// value at the first longitude of the sweep (captured on the way); seam_f
-// and seam_r: the seam coefficients of both directions.
-template <int kRG, int G>
-struct SweepMem {
-  double *val;      // [kRG][G][Rp]
-  double2 *cof;     // [kRG][G][Rp]
-  double *stage;    // [2][G][Rp]
-  double *edge;     // [Rp] by row
-  double *seam_f;   // [Rp] by row: lu/dg at longitude np-1
-  double *seam_r;   // [Rp] by row: ll/dg at longitude 0
-  uint64_t *bar;    // [kRG]
-  int Rp;
-
-  // lane 0: fetch diagonals d0 .. d0 + G - 1 of (va, vb) into the slot of group n
-  __device__ __forceinline__ void issue(unsigned n, const double *va, const double2 *vb,
-                                        size_t d0) const {
-    const unsigned slot = n % kRG;
-    const unsigned bv = (unsigned)(G * Rp) * 8u, bc = (unsigned)(G * Rp) * 16u;
-    const unsigned b = smem_u32(bar + slot);
-    // relaxed: the copies carry the data, the arrival orders nothing else
-    asm volatile("mbarrier.arrive.expect_tx.relaxed.cta.shared::cta.b64 _, [%0], %1;" ::"r"(b),
-                 "r"(bv + bc)
-                 : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-        "[%3];" ::"r"(smem_u32(val + (size_t)slot * G * Rp)),
-        "l"(va + d0 * Rp), "r"(bv), "r"(b)
-        : "memory");
-    asm volatile(
-        "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, "
-        "[%3];" ::"r"(smem_u32(cof + (size_t)slot * G * Rp)),
-        "l"(vb + d0 * Rp), "r"(bc), "r"(b)
-        : "memory");
-  }
-  // wait (bounded) until group n's slot is filled
-  __device__ __forceinline__ bool wait(unsigned n, unsigned limit = kSpinLimit) const {
-    const unsigned b = smem_u32(bar + n % kRG), parity = (n / kRG) & 1u;
-    for (unsigned it = 0;; ++it) {
-      unsigned ok;
-      asm volatile(
-          "{\n .reg .pred p;\n mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-          " selp.u32 %0, 1, 0, p;\n}"
-          : "=r"(ok)
-          : "r"(b), "r"(parity)
-          : "memory");
-      if (ok) return true;
-      if (it >= limit) return false;
-    }
-  }
-};
-
-template <int N>
-__device__ __forceinline__ void bulk_wait_read() {
-  asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory");
-}
-__device__ __forceinline__ void bulk_wait_all() {
-  asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
-}
-
-// The sweep warp gave up waiting for a copy: record it, then wait (again
-// bounded) for the groups it still has in flight, n0 .. n1 - 1.
-template <int kRG, int G>
-__device__ __noinline__ void sweep_abort(const TSys &S, const SweepMem<kRG, G> &sm, unsigned n0,
-                                         unsigned n1) {
-  if ((threadIdx.x & 31) == 0) {
-    atomicExch(S.fault, 1);
-    bulk_wait_all();
-  }
-  for (unsigned n = n0; n < n1; ++n) sm.wait(n, kDrainLimit);
-}
-
-// One wavefront sweep by one warp.  Step s handles anti-diagonal
-// diag(s) (s for the forward sweep, Rp + np - 2 - s for the reverse).  Lane
-// l holds rows l M + m, m < M, as chains:
-//   v(r) = a(r) - c.y(r) v_prev(r) - c.x(r) n(r)
-// where a is the value stream, c the coefficient pair, v_prev the row's
-// previous value (the west / east neighbour) and n the previous step's
-// value of the row below / above -- chain m -+ 1 of the same lane, or for
-// the lane's first / last chain the neighbouring lane's last / first chain
-// by warp shuffle.  Off-grid points and padding rows read zeros and produce
-// exact zeros.  Work is grouped G steps at a time: one pair of bulk loads,
-// one wait and one bulk store per group, and every load of a step is issued
-// before any store.  The seam term of the one point per step on the seam
-// longitude is folded into that point's value in the ring, a group ahead,
-// from the row's captured edge value (groups of G need the seam
-// np - 1 >= 2 G steps after the edge).
-//
-// Forward (nonorthogonal_mi.c:910-937), on D^-1-scaled rows:
-//   fw = in/dg - (lo/dg) fw(r-1, j) - (ll/dg) fw(r, j-1) - (lu/dg) fw(r, 0)|j=np-1
-// Reverse (nonorthogonal_mi.c:939-964):
-//   out = fw - (up/dg) out(r+1, j) - (lu/dg) out(r, j+1) - (ll/dg) out(r, np-1)|j=0
-// with the pole sum sum_j pe_j out(1, j) accumulated from row 0.
-template <int M, int kRG, int G, bool kReverse>
-__device__ __forceinline__ bool sweep(const TSys &S, const double *__restrict__ in,
-                                      double *__restrict__ out, const SweepMem<kRG, G> &sm,
-                                      unsigned &gn, const double *pe_s, double boundary,
-                                      double &psum) {
-  const int lane = threadIdx.x & 31, R = S.R, Rp = S.Rp, np = S.np;
-  const int dmax = Rp + np - 2;
-  const int ngroups = (Rp + np - 1 + G - 1) / G;  // steps padded to whole groups
-  const double2 *coef = kReverse ? S.cb : S.cf;
-  const double *seam = kReverse ? sm.seam_r : sm.seam_f;
-  // lowest column of group k, and the slot index of step u of a group
-  auto group_d0 = [&](int k) {
-    return (size_t)(kPad + (kReverse ? dmax - (k * G + G - 1) : k * G));
-  };
-  auto sub = [&](int u) { return kReverse ? G - 1 - u : u; };
-  // seam point of step s: row s - (np - 1) (forward) / dmax - s (reverse);
-  // edge point: row s at longitude 0 / row Rp - 1 - s at longitude np - 1
-  auto seam_row = [&](int s) { return kReverse ? dmax - s : s - (np - 1); };
-  auto edge_row = [&](int s) { return kReverse ? Rp - 1 - s : s; };
-  auto pos = [&](int r) { return (r % M) * 32 + r / M; };
-  double v[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) v[m] = 0.0;
-  psum = 0.0;
-  // operands (value, coefficient pair) of step u of group k, for this lane's chains
-  double ca[M];
-  double2 cc[M];
-  auto load = [&](int k, int u, double (&a)[M], double2 (&c)[M]) {
-    const size_t base = ((size_t)((gn + k) % kRG) * G + sub(u)) * Rp + lane;
-    const double *__restrict__ rv = sm.val + base;
-    const double2 *__restrict__ rc = sm.cof + base;
-#pragma unroll
-    for (int m = 0; m < M; ++m) {
-      a[m] = rv[32 * m];
-      c[m] = rc[32 * m];
-    }
-  };
-  // the value stream was written through the generic proxy (a vector phase,
-  // or the forward sweep's drained stores) and is read by bulk copies
-  if (lane == 0) bulk_wait_all();
-  asm volatile("fence.proxy.async;" ::: "memory");
-  __syncwarp();
-  if (lane == 0)
-    for (int k = 0; k < kRG - 1 && k < ngroups; ++k) sm.issue(gn + k, in, coef, group_d0(k));
-  bool ok = true;
-  if (lane < G) ok = sm.wait(gn);  // group 0 has no seam point
-  for (int k = 0; k < ngroups; ++k) {
-    const unsigned n = gn + k;
-    if (!__all_sync(0xffffffffu, ok)) {
-      sweep_abort(S, sm, n, gn + (unsigned)min(k + kRG - 1, ngroups));
-      gn += ngroups;
-      return false;
-    }
-    if (lane == 0) {
-      if (k + kRG - 1 < ngroups) sm.issue(n + kRG - 1, in, coef, group_d0(k + kRG - 1));
-      bulk_wait_read<1>();  // the stage half of this group is free again
-    }
-    // lanes u < G: wait for the next group and fold its seam terms
-    if (lane < G && k + 1 < ngroups) {
-      ok = sm.wait(n + 1);
-      const int r = seam_row((k + 1) * G + lane);
-      if (ok && r >= 0 && r < R) {
-        double *p = sm.val + ((size_t)((n + 1) % kRG) * G + sub(lane)) * Rp + pos(r);
-        *p = fma(-seam[r], sm.edge[r], *p);
-      }
-    }
-    __syncwarp();
-    if (k == 0) load(0, 0, ca, cc);
-    double *gs = sm.stage + (size_t)(k & 1) * G * Rp;
-#pragma unroll
-    for (int u = 0; u < G; ++u) {
-      // operands of the next step, loaded before this step computes and stores
-      double na[M];
-      double2 nc[M];
-      if (u + 1 < G)
-        load(k, u + 1, na, nc);
-      else if (k + 1 < ngroups)
-        load(k + 1, 0, na, nc);
-      double nb[M];
-      if (kReverse) {
-        const double x = __shfl_sync(0xffffffffu, v[0], (lane + 1) & 31);
-        nb[M - 1] = lane == 31 ? 0.0 : x;  // no row above the top one
-#pragma unroll
-        for (int m = 0; m + 1 < M; ++m) nb[m] = v[m + 1];
-      } else {
-        const double x = __shfl_sync(0xffffffffu, v[M - 1], (lane + 31) & 31);
-        nb[0] = lane == 0 ? boundary : x;  // the pole below row 0
-#pragma unroll
-        for (int m = 1; m < M; ++m) nb[m] = v[m - 1];
-      }
-#pragma unroll
-      for (int m = 0; m < M; ++m) v[m] = fma(-cc[m].x, nb[m], fma(-cc[m].y, v[m], ca[m]));
-      if (kReverse) {
-        const int d = dmax - (k * G + u);
-        psum = fma(pe_s[d < 0 ? 0 : d < np ? d : np - 1], v[0], psum);
-      }
-      double *__restrict__ st = gs + sub(u) * Rp + lane;
-#pragma unroll
-      for (int m = 0; m < M; ++m) st[32 * m] = v[m];
-#pragma unroll
-      for (int m = 0; m < M; ++m) {
-        ca[m] = na[m];
-        cc[m] = nc[m];
-      }
-    }
-    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    __syncwarp();
-    if (lane < G) {
-      // edge capture for this group's steps
-      const int re = edge_row(k * G + lane);
-      if (re >= 0 && re < R) sm.edge[re] = gs[sub(lane) * Rp + pos(re)];
-    }
-    __syncwarp();  // captured edges are visible to the seam folds of later groups
-    if (lane == 0) {
-      asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
-                       out + group_d0(k) * Rp),
-                   "r"(smem_u32(gs)), "r"((unsigned)(G * Rp) * 8u)
-                   : "memory");
-      asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-    }
-  }
-  gn += ngroups;
-  if (lane == 0) {
-    bulk_wait_all();
-    asm volatile("fence.proxy.async;" ::: "memory");
-  }
-  __syncwarp();
-  return true;
 }
 
 // Band-pipelined sweeps.  CTA b of the cluster owns the interior rows
@@ -460,6 +246,261 @@ __device__ __forceinline__ bool inbox_take(const double *p, double &v) {
   return false;
 }
 
+// (no memory clobber: the ring slots a copy fills are read after the wait
+// that follows it in program order)
+__device__ __forceinline__ void copy16(unsigned dst, const void *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
+}
+
+// Inboxes carry kInboxPad slots before the first longitude and as many and a
+// group after the last, so a sending lane stores its off-grid steps too
+// (columns -7 .. np + 37 less the lane), without a test.
+constexpr int kInboxPad = 32;
+__host__ __device__ constexpr int inbox_len(int np) { return np + 2 * kInboxPad + kGroup; }
+
+// Shared memory of the sweep warps of one CTA: per warp a prefetch ring and
+// the two inboxes (the row below the block for the forward sweep, above it
+// for the reverse).  Block 0 receives no row below: the pole edges by column
+// (zero off the grid) are kept in its place.
+struct WaveMem {
+  unsigned char *ring;    // [warps][kRing][kStepBytes]
+  double *inf, *inr;      // [warps][inbox_len]
+  double *pe;             // [inbox_len], CTA 0
+};
+
+// What a sweep warp holds between steps.
+struct WaveState {
+  double v0, v1;          // the lane's two rows at the previous step
+  double edge0, edge1;    // ... at the sweep's first longitude
+  double seam0, seam1;    // seam coefficients of the two rows
+  double psum;
+};
+// A step's operands of the lane: two values, two coefficient pairs.
+struct WaveOperands {
+  double2 a, c0, c1;
+  __device__ __forceinline__ void load(const unsigned char *at) {
+    a = *reinterpret_cast<const double2 *>(at);
+    c0 = *reinterpret_cast<const double2 *>(at + 512);
+    c1 = *reinterpret_cast<const double2 *>(at + 1024);
+  }
+};
+// Where the copies of a group's steps come from and go to.
+struct WaveCopy {
+  const double *a;
+  const double2 *c;
+  unsigned to;
+};
+constexpr int kEmptyHigh = (int)(kEmpty >> 32);
+
+// The kGroup steps of one group; col0 is the first step's column, vo and
+// to_next its output and neighbour inbox addresses.  kEdgy: the group holds a
+// point on the first or last longitude; kPole: block 0 of the reverse sweep.
+//
+// A step is a chain of some 50 cycles (a shuffle, a select and two
+// multiply-adds) with few instructions of its own, so everything else is
+// placed between the steps: the operands of four steps on are loaded from the
+// ring (o[u % 4]), those of 24 steps on are copied into it, and halfway
+// through the linking lane looks at the neighbouring block's row of the next
+// group (next_e).
+template <bool kReverse, bool kEdgy, bool kPole>
+__device__ __forceinline__ void wave_group(WaveState &s, WaveOperands (&o)[4],
+                                           const unsigned char *here,
+                                           const unsigned char *there, const WaveCopy &cp,
+                                           bool copying, const double (&e)[kGroup],
+                                           double (&next_e)[kGroup], const double *next_in,
+                                           bool linked, bool link, unsigned send, int col0,
+                                           int np, double *vo, unsigned to_next,
+                                           const double *pe) {
+  constexpr int dir = kReverse ? -1 : 1;
+  const int lane = threadIdx.x & 31;
+#pragma unroll
+  for (int u = 0; u < kGroup; ++u) {
+    const int j = col0 + dir * u - lane;
+    double t0 = o[u % 4].a.x, t1 = o[u % 4].a.y;
+    if (kEdgy && j == (kReverse ? 0 : np - 1)) {
+      t0 = fma(-s.seam0, s.edge0, t0);
+      t1 = fma(-s.seam1, s.edge1, t1);
+    }
+    double x = kReverse ? __shfl_down_sync(0xffffffffu, s.v0, 1)
+                        : __shfl_up_sync(0xffffffffu, s.v1, 1);
+    t0 = fma(-o[u % 4].c0.y, s.v0, t0);
+    t1 = fma(-o[u % 4].c1.y, s.v1, t1);
+    const double c0x = o[u % 4].c0.x, c1x = o[u % 4].c1.x;
+    o[u % 4].load((u + 4 < kGroup ? here : there) + ((u + 4) % kGroup) * kStepBytes);
+    if (copying) {
+      copy16(cp.to + u * kStepBytes, cp.a + dir * u * kBlockRows);
+      copy16(cp.to + u * kStepBytes + 512, cp.c + dir * u * kBlockRows);
+      copy16(cp.to + u * kStepBytes + 1024, cp.c + dir * u * kBlockRows + 32);
+    }
+    x = link ? e[u] : x;
+    if (kReverse) {
+      s.v1 = fma(-c1x, x, t1);
+      s.v0 = fma(-c0x, s.v1, t0);
+    } else {
+      s.v0 = fma(-c0x, x, t0);
+      s.v1 = fma(-c1x, s.v0, t1);
+    }
+    if (kEdgy && j == (kReverse ? np - 1 : 0)) {
+      s.edge0 = s.v0;
+      s.edge1 = s.v1;
+    }
+    // (predicated, not branched around: one lane sends)
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n"
+        " @p st.relaxed.cluster.shared::cluster.b64 [%0], %1;\n}" ::"r"(
+            to_next + (unsigned)(dir * u * 8)),
+        "d"(kReverse ? s.v0 : s.v1), "r"(send));
+    *reinterpret_cast<double2 *>(vo + dir * u * kBlockRows) = make_double2(s.v0, s.v1);
+    if (kPole) s.psum = fma(pe[dir * u], s.v0, s.psum);
+    if (linked && u == kGroup / 2) {
+#pragma unroll
+      for (int q = 0; q < kGroup; ++q) next_e[q] = inbox_peek(next_in + dir * q);
+    }
+  }
+}
+
+// One sweep of block w by one warp (see the top of the file).  Step t
+// handles column t (forward) or np + 30 - t (reverse) of the block:
+//   forward  v = a - (lo/dg) v(r-1, j) - (ll/dg) v(r, j-1) [- (lu/dg) v(r, 0) at j = np-1]
+//   reverse  v = fw - (up/dg) v(r+1, j) - (lu/dg) v(r, j+1) [- (ll/dg) v(r, np-1) at j = 0]
+// (nonorthogonal_mi.c:910-964); off-grid points read zeros and produce zeros.
+// psum accumulates the pole edge sum over row 0 (block 0).  Returns false
+// when a value of the neighbouring block never arrived: the fault is recorded
+// and the remaining steps use what the inbox holds.
+template <bool kReverse>
+__device__ __noinline__ bool wave_sweep(const TSys &S, const double *__restrict__ in,
+                                        double *__restrict__ out, const WaveMem &wm,
+                                        int slot, int w, int csize, double boundary,
+                                        double &psum) {
+  // groups copied beyond the current one; the next one has landed when a
+  // group begins
+  constexpr int kAhead = kRing / kGroup - 1;
+  static_assert(kAhead >= 2, "the ring holds the current, the next and a copied group");
+  constexpr int dir = kReverse ? -1 : 1;
+  const int lane = threadIdx.x & 31, np = S.np;
+  const int ngroups = (np + 31 + kGroup - 1) / kGroup;
+  const int start = kReverse ? np + 30 : 0;   // first column
+  const size_t base = ((size_t)w * S.cols + kPad + start) * kBlockRows;
+  WaveCopy cp{in + base + 2 * lane, (kReverse ? S.cb : S.cf) + base + lane, 0u};
+  double *vo = out + base + 2 * lane;
+  unsigned char *ring = wm.ring + (size_t)slot * kRing * kStepBytes + lane * 16;
+  const unsigned ring_at = smem_u32(ring);
+  auto slot_of = [&](int g) { return (unsigned)((g * kGroup) & (kRing - 1)) * (unsigned)kStepBytes; };
+  WaveState s{};
+  {
+    // the other sweep's pair at this sweep's last longitude
+    const double2 *sc = (kReverse ? S.cf : S.cb) +
+                        ((size_t)w * S.cols + kPad + lane + (kReverse ? 0 : np - 1)) * kBlockRows +
+                        lane;
+    s.seam0 = sc[0].y;
+    s.seam1 = sc[32].y;
+  }
+  const bool from = kReverse ? w + 1 < S.blocks : w > 0;
+  const bool link = kReverse ? lane == 31 : lane == 0;
+  const bool send = kReverse ? lane == 0 && w > 0 : lane == 31 && w + 1 < S.blocks;
+  double *boxes = kReverse ? wm.inr : wm.inf;
+  double *inbox = boxes + (size_t)slot * inbox_len(np) + kInboxPad;  // by longitude
+  unsigned to_next = 0u;   // the sending lane's longitude is its column less its lane
+  if (send) {
+    const int to = kReverse ? w - 1 : w + 1;
+    to_next = cluster_addr(boxes + (size_t)(to / csize) * inbox_len(np) + kInboxPad + start -
+                               lane, to % csize);
+  }
+  const bool pole = kReverse && w == 0;
+  const double *pe = wm.pe + kInboxPad + start;
+  const double fixed = kReverse ? 0.0 : boundary;
+  bool ok = true;
+  auto copy_group = [&]() {
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) {
+      copy16(cp.to + u * kStepBytes, cp.a + dir * u * kBlockRows);
+      copy16(cp.to + u * kStepBytes + 512, cp.c + dir * u * kBlockRows);
+      copy16(cp.to + u * kStepBytes + 1024, cp.c + dir * u * kBlockRows + 32);
+    }
+  };
+  auto next_copy = [&]() {
+    cp.a += dir * kGroup * kBlockRows;
+    cp.c += dir * kGroup * kBlockRows;
+  };
+#pragma unroll
+  for (int g = 0; g < kAhead; ++g) {
+    if (g < ngroups) {
+      cp.to = ring_at + slot_of(g);
+      copy_group();
+      next_copy();
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  }
+  asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+  WaveOperands o[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) o[u].load(ring + u * kStepBytes);
+  // the linking lane's first longitude of group k in the neighbour's row
+  auto row_at = [&](int k) { return start + dir * k * kGroup - (kReverse ? 31 : 0); };
+  double e[kGroup], next_e[kGroup];
+#pragma unroll
+  for (int u = 0; u < kGroup; ++u)
+    next_e[u] = from ? __longlong_as_double((long long)kEmpty) : fixed;
+  for (int k = 0; k < ngroups; ++k) {
+    const int col0 = start + dir * k * kGroup;
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) e[u] = next_e[u];
+    // the next group's operands have landed too
+    asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 2) : "memory");
+    if (from) {
+      const int j0 = row_at(k);
+      // longitudes off the grid are not waited for (their points are zero)
+      auto missing = [&]() {
+        bool any = false;
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u)
+          any = any || (__double2hiint(e[u]) == kEmptyHigh &&
+                        (unsigned)(j0 + dir * u) < (unsigned)np);
+        return any && link;
+      };
+      unsigned tries = 0;
+      while (__any_sync(0xffffffffu, missing()) && ok) {
+#pragma unroll
+        for (int u = 0; u < kGroup; ++u) e[u] = inbox_peek(inbox + j0 + dir * u);
+        ok = ++tries < kInboxSpinLimit;
+      }
+#pragma unroll
+      for (int u = 0; u < kGroup; ++u)
+        if (__double2hiint(e[u]) == kEmptyHigh) e[u] = 0.0;
+    }
+    const unsigned char *here = ring + slot_of(k), *there = ring + slot_of(k + 1);
+    cp.to = ring_at + slot_of(k + kAhead);
+    const bool copying = k + kAhead < ngroups, linked = from && k + 1 < ngroups;
+    const double *next_in = inbox + row_at(k + 1);
+    // the only groups with a point on the first or the last longitude
+    const int last = col0 + dir * (kGroup - 1);
+    if (pole)
+      wave_group<kReverse, true, true>(s, o, here, there, cp, copying, e, next_e, next_in,
+                                       linked, link, send, col0, np, vo, to_next, pe);
+    else if (min(col0, last) <= 31 || max(col0, last) >= np - 1)
+      wave_group<kReverse, true, false>(s, o, here, there, cp, copying, e, next_e, next_in,
+                                        linked, link, send, col0, np, vo, to_next, pe);
+    else
+      wave_group<kReverse, false, false>(s, o, here, there, cp, copying, e, next_e, next_in,
+                                         linked, link, send, col0, np, vo, to_next, pe);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    next_copy();
+    vo += dir * kGroup * kBlockRows;
+    to_next += (unsigned)(dir * kGroup * 8);
+    pe += dir * kGroup;
+  }
+  psum = s.psum;
+  // every value of the inbox has been taken: mark it empty for the next sweep
+  __syncwarp();
+  if (from)
+    for (int j = lane; j < np; j += 32) inbox[j] = __longlong_as_double((long long)kEmpty);
+  if (!ok && lane == 0) atomicExch(S.fault, 1);
+  // the reverse sweep's copies read what this lane stored here
+  __threadfence();
+  __syncwarp();
+  return ok;
+}
+
 // One sweep of band b (rows r0 .. r0 + hb - 1) by warp 0 of its CTA, the
 // recurrences of sweep() on the same D^-1-scaled operands:
 //   forward  v = val - (lo/dg) v(r-1, j) - (ll/dg) v(r, j-1) [- (lu/dg) v(r, 0) at j = np-1]
@@ -487,9 +528,8 @@ __device__ __noinline__ bool band_sweep(const TSys &S, const BandMem &bm, int b,
       (kReverse ? lane == 0 : lane == hb - 1) && (kReverse ? b > 0 : b + 1 < nbands);
   double *inbox = kReverse ? bm.inr : bm.inf;
   const unsigned dst = send ? cluster_addr(inbox, kReverse ? b - 1 : b + 1) : 0u;
-  // the row's first point in the skewed output: (kPad + r + j) Rp + row_pos(r)
-  double *orow =
-      out + (size_t)(kPad + r0 + lane) * S.Rp + (row_on ? row_pos(S.Rp, r0 + lane) : 0);
+  // the row's first point in the skewed output
+  double *orow = out + (row_on ? sidx(S.cols, r0 + lane, 0) : 0);
   const double fixed = kReverse ? 0.0 : boundary;  // pole below row 0; nothing above row R-1
   const bool pole_row = kReverse && b == 0 && lane == 0;
   bool ok = true;
@@ -517,7 +557,7 @@ __device__ __noinline__ bool band_sweep(const TSys &S, const BandMem &bm, int b,
       v = fma(-c.x, x, fma(-c.y, v, a));
       if (j == (kReverse ? np - 1 : 0)) edge = v;
       if (kReverse)
-        orow[(size_t)j * S.Rp] = v;
+        orow[(size_t)j * kBlockRows] = v;
       else
         val[slot] = v;
       if (pole_row) psum = fma(bm.pe[j], v, psum);
@@ -537,12 +577,12 @@ __device__ __noinline__ bool band_sweep(const TSys &S, const BandMem &bm, int b,
 // (A p) at a grid point of the skewed layout (nonorthogonal_mi.c:867-900).
 __device__ __forceinline__ double apply_at(const TSys &S, const double *p, size_t k, int row,
                                            int j, double pole) {
-  const int R = S.R, Rp = S.Rp, np = S.np;
-  const size_t q = (size_t)row_pos(Rp, row);
-  const double lv = row == 0 ? pole : p[k - q - Rp + row_pos(Rp, row - 1)];
-  const double uv = row + 1 < R ? p[k - q + Rp + row_pos(Rp, row + 1)] : 0.0;
-  const size_t kw = j == 0 ? k + (size_t)(np - 1) * Rp : k - Rp;
-  const size_t ke = j + 1 == np ? k - (size_t)(np - 1) * Rp : k + Rp;
+  const int np = S.np;
+  const size_t wrap = (size_t)(np - 1) * kBlockRows;
+  const double lv = row == 0 ? pole : p[below(S.cols, k, row, j)];
+  const double uv = row + 1 < S.R ? p[above(S.cols, k, row, j)] : 0.0;
+  const size_t kw = j == 0 ? k + wrap : k - kBlockRows;
+  const size_t ke = j + 1 == np ? k - wrap : k + kBlockRows;
   return S.dg[k] * p[k] + S.lo[k] * lv + S.up[k] * uv + S.ll[k] * p[kw] + S.lu[k] * p[ke];
 }
 
@@ -561,45 +601,39 @@ struct Acc {
   double v[N] = {};
 };
 
-// Row and longitude of skewed index k; false off the grid and on padding rows.
-__device__ __forceinline__ bool locate(int R, int Rp, int np, unsigned k, int &row, int &j) {
-  const unsigned col = k / (unsigned)Rp;
-  row = pos_row(Rp, (int)(k - col * (unsigned)Rp));
-  j = (int)col - kPad - row;
-  return row < R && (unsigned)j < (unsigned)np;
+// Row and longitude of index k; false off the grid and on padding rows.
+__device__ __forceinline__ bool locate(const TSys &S, unsigned k, int &row, int &j) {
+  const unsigned q = S.loc[k];
+  row = (int)(q >> 13) - 1;
+  j = (int)(q & 8191u);
+  return q != 0u;
 }
 
-// Dynamic shared memory of a launch: the sweep ring (kRG G diagonals of
-// Rp values and Rp coefficient pairs), 2 G staged output diagonals, three
-// row tables and the pole-edge table.
-size_t tensor_smem(int kRG, int G, int Rp, int np) {
-  return ((size_t)kRG * G * Rp * 3 + (size_t)(2 * G + 3) * Rp + (size_t)np) * sizeof(double);
+// Dynamic shared memory of a launch: the rings and inboxes of the CTA's
+// sweep warps.
+size_t tensor_smem(int warps, int np) {
+  return (size_t)warps * (kRing * kStepBytes + 2 * inbox_len(np) * sizeof(double));
 }
 
-template <int M, int kRG, int kG>
 __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
   constexpr int kT = kThreads, kWarps = kT / 32;
-  constexpr int kB = 8;  // grid points a thread loads per batch
+  constexpr int kB = 5;  // grid points a thread loads per batch
   extern __shared__ __align__(128) double dyn_smem[];
-  __shared__ uint64_t ring_bar[kRG];
   __shared__ double wbuf[kWarps * kSlotWidth];
   __shared__ double slots[kSlots * kMaxCluster * kSlotWidth];
   __shared__ double bcast[2];
   cg::cluster_group cl = cg::this_cluster();
   const int rank = (int)cl.block_rank(), csize = (int)cl.num_blocks();
   Reducer<kWarps> red{wbuf, slots, 0, rank, csize};
-  const int np = S.np, nt = S.nt, R = S.R, Rp = S.Rp, t = threadIdx.x, lane = t & 31,
+  const int np = S.np, nt = S.nt, R = S.R, cols = S.cols, t = threadIdx.x, lane = t & 31,
             warp = t >> 5;
-  SweepMem<kRG, kG> sm;
-  sm.val = dyn_smem;
-  sm.cof = reinterpret_cast<double2 *>(dyn_smem + (size_t)kRG * kG * Rp);
-  sm.stage = dyn_smem + (size_t)kRG * kG * Rp * 3;
-  sm.edge = sm.stage + (size_t)2 * kG * Rp;
-  sm.seam_f = sm.edge + Rp;
-  sm.seam_r = sm.seam_f + Rp;
-  sm.bar = ring_bar;
-  sm.Rp = Rp;
-  double *pe_s = sm.seam_r + Rp;
+  // sweep warps of a CTA: block w runs on CTA w mod csize, warp w / csize
+  const int sweepers = (S.blocks + csize - 1) / csize;
+  WaveMem wm;
+  wm.ring = reinterpret_cast<unsigned char *>(dyn_smem);
+  wm.inf = dyn_smem + (size_t)sweepers * kRing * (kStepBytes / sizeof(double));
+  wm.inr = wm.inf + (size_t)sweepers * inbox_len(np);
+  wm.pe = wm.inf;
   // the band schedule's tables share the dynamic shared memory
   BandMem bm;
   bm.h = S.band;
@@ -612,16 +646,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     bm.inr = bm.inf + np;
     bm.pe = bm.inr + np;
   }
-  if (S.band)
-    for (int j = threadIdx.x; j < np; j += kT)
-      bm.inf[j] = bm.inr[j] = __longlong_as_double((long long)kEmpty);
-  if (rank == 0 && t == 0) {
-    for (int q = 0; q < kRG; ++q)
-      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_u32(ring_bar + q))
-                   : "memory");
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    *S.fault = 0;
+  {
+    double *inboxes = S.band ? bm.inf : wm.inf;
+    const int n = 2 * (S.band ? np : sweepers * inbox_len(np));
+    for (int j = threadIdx.x; j < n; j += kT)
+      inboxes[j] = __longlong_as_double((long long)kEmpty);
   }
+  if (rank == 0 && t == 0) *S.fault = 0;
   const unsigned g = (unsigned)(rank * kT + t), G = (unsigned)(csize * kT);
   const bool lead = g == 0;
   const unsigned nq = (unsigned)(R * np);
@@ -663,15 +694,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     const double up = -upper + dfp / (2.0 * S.dth);
     const double ll = -llo + dft / (2.0 * S.dph);
     const double lu = -lup - dft / (2.0 * S.dph);
-    const size_t k = sidx(Rp, row, j);
+    const size_t k = sidx(cols, row, j), kc = cidx(cols, row, j);
+    S.loc[k] = (unsigned)(row + 1) << 13 | (unsigned)j;
+    S.wt[k] = 1.0 / Rw.s;
     S.dg[k] = d;
     S.lo[k] = lo;
     S.up[k] = up;
     S.ll[k] = ll;
     S.lu[k] = lu;
     S.rdg[k] = 1.0 / d;
-    S.cf[k] = make_double2(lo / d, ll / d);
-    S.cb[k] = make_double2(up / d, lu / d);
+    S.cf[kc] = make_double2(lo / d, ll / d);
+    S.cb[kc] = make_double2(up / d, lu / d);
     // right-hand side and initial guess (nonorthogonal_mi.c:999-1029)
     const double f = S.fac[full];
     const double u = S.neg_r2 * f * Rw.inc;
@@ -710,7 +743,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     for (int q = t; q < slots; q += kT) {
       const int d = q / h, l = q - d * h, j = d - l;
       const bool on = l < hb && j >= 0 && j < np;
-      const size_t k = on ? sidx(Rp, r0 + l, j) : 0;
+      const size_t k = on ? cidx(cols, r0 + l, j) : 0;
       bm.cf[q] = on ? S.cf[k] : make_double2(0.0, 0.0);
       bm.cb[q] = on ? S.cb[k] : make_double2(0.0, 0.0);
       bm.val[q] = 0.0;
@@ -718,10 +751,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     if (rank == 0)
       for (int j = t; j < np; j += kT) bm.pe[j] = S.pe[j];
   } else if (rank == 0) {
-    for (int j = t; j < np; j += kT) pe_s[j] = S.pe[j];
-    for (int r = t; r < Rp; r += kT) {
-      sm.seam_f[r] = r < R ? S.cb[sidx(Rp, r, np - 1)].y : 0.0;
-      sm.seam_r[r] = r < R ? S.cf[sidx(Rp, r, 0)].y : 0.0;
+    for (int q = t; q < inbox_len(np); q += kT) {
+      const int j = q - kInboxPad;
+      wm.pe[q] = j >= 0 && j < np ? S.pe[j] : 0.0;
     }
   }
   __syncthreads();
@@ -743,9 +775,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
       for (int b = 0; b < kB; ++b) {
         const unsigned k = k0 + b * G;
         int row = 0, j = 0;
-        on[b] = k < core1 && locate(R, Rp, np, k, row, j);
+        on[b] = k < core1 && locate(S, k, row, j);
         r[b] = on[b] ? S.rhs[k] - apply_at(S, S.x, k, row, j, x0) : 0.0;
-        wr[b] = on[b] ? S.rows[row + 1].s : 1.0;
+        wr[b] = on[b] ? S.wt[k] : 0.0;
         xr[b] = on[b] && row == 0 ? S.pe[j] * S.x[k] : 0.0;
       }
 #pragma unroll
@@ -756,7 +788,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
         S.shd[k] = r[b];
         S.srch[k] = 0.0;
         S.as[k] = 0.0;
-        const double wv = r[b] / wr[b];
+        const double wv = r[b] * wr[b];
         a[0] += wv * wv;
         a[1] += r[b] * r[b];
         a[2] += xr[b];
@@ -786,7 +818,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
       for (int b = 0; b < kB; ++b) {
         const unsigned k = k0 + b * G;
         int row = 0, j = 0;
-        on[b] = k < core1 && locate(R, Rp, np, k, row, j);
+        on[b] = k < core1 && locate(S, k, row, j);
         av[b] = on[b] ? apply_at(S, p, k, row, j, p0) : 0.0;
         o[b] = on[b] ? (acc.n == 1 ? S.shd[k] : S.mid[k]) : 0.0;
       }
@@ -822,16 +854,17 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
   int conv = initial <= target;
   double rho_prev = 1.0, alpha = 1.0, omega = 1.0;
   const int max_iter = S.max_iter < kMaxIterations ? S.max_iter : kMaxIterations;
-  const bool sweeper = rank == 0 && warp == 0;
-  unsigned gn = 0;  // running group count of the sweep warp's prefetch ring
-  // SSOR of in (D^-1-scaled, pole at in[0]) into out, by the sweep warp
+  // SSOR of in (D^-1-scaled, pole at in[0]) into out, one warp per block
+  const bool sweeper = warp < sweepers && rank + warp * csize < S.blocks;
   auto ssor = [&](const double *in, double *out) {
+    const int w = rank + warp * csize;
+    const double in0 = w == 0 ? in[0] : 0.0;
     double psum = 0.0;
-    if (lane == 0) S.fw[0] = in[0];
-    if (sweep<M, kRG, kG, false>(S, in, S.fw, sm, gn, pe_s, in[0], psum) &&
-        sweep<M, kRG, kG, true>(S, S.fw, out, sm, gn, pe_s, 0.0, psum) && lane == 0) {
+    if (wave_sweep<false>(S, in, S.fw, wm, warp, w, csize, in0, psum) &&
+        wave_sweep<true>(S, S.fw, out, wm, warp, w, csize, 0.0, psum) && w == 0 &&
+        lane == 0) {
       // pole (nonorthogonal_mi.c:958-963): (dg0 fw0 + sum pe_j out(1, j)) / dg0
-      out[0] = (dg0 * S.fw[0] + psum) / dg0;
+      out[0] = (dg0 * in0 + psum) / dg0;
       *S.pole_sum = psum;
     }
   };
@@ -842,7 +875,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     const double in0 = in[0];
     for (int q = t; q < hb * np; q += kT) {
       const int l = q / np, j = q - l * np;
-      bm.val[(size_t)(j + l) * h + l] = in[sidx(Rp, r0 + l, j)];
+      bm.val[(size_t)(j + l) * h + l] = in[sidx(cols, r0 + l, j)];
     }
     __syncthreads();
     if (warp == 0 && hb > 0) {
@@ -896,8 +929,8 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
 #pragma unroll
             for (int q = 0; q < 4; ++q) cf[b][q] = nb[b][q] = 0.0;
             if (!on[b]) continue;
-            const size_t k = sidx(Rp, row, j);
-            const size_t q = (size_t)row_pos(Rp, row);
+            const size_t k = sidx(cols, row, j);
+            const size_t wrap = (size_t)(np - 1) * kBlockRows;
             const int jm = j == 0 ? np - 1 : j - 1, jp = j + 1 == np ? 0 : j + 1;
             kk[b] = k;
             v[b] = dir == 0 ? in[k] : fw[k];
@@ -906,10 +939,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
             const int cn[4] = {row == 0 ? -1 : tcolor(row - 1, j, np),
                                row + 1 < R ? tcolor(row + 1, j, np) : c,
                                tcolor(row, jm, np), tcolor(row, jp, np)};
-            const size_t kn[4] = {row == 0 ? 0 : k - q - Rp + row_pos(Rp, row - 1),
-                                  row + 1 < R ? k - q + Rp + row_pos(Rp, row + 1) : k,
-                                  j == 0 ? k + (size_t)(np - 1) * Rp : k - Rp,
-                                  j + 1 == np ? k - (size_t)(np - 1) * Rp : k + Rp};
+            const size_t kn[4] = {row == 0 ? 0 : below(cols, k, row, j),
+                                  row + 1 < R ? above(cols, k, row, j) : k,
+                                  j == 0 ? k + wrap : k - kBlockRows,
+                                  j + 1 == np ? k - wrap : k + kBlockRows};
             const double *co[4] = {S.lo, S.up, S.ll, S.lu};
 #pragma unroll
             for (int e = 0; e < 4; ++e) {
@@ -933,7 +966,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     }
     // pole (nonorthogonal_mi.c:958-963): (dg0 fw0 + sum pe_j out(1, j)) / dg0
     double ps[1] = {0.0};
-    for (unsigned jj = g; jj < (unsigned)np; jj += G) ps[0] += S.pe[jj] * out[sidx(Rp, 0, jj)];
+    for (unsigned jj = g; jj < (unsigned)np; jj += G) ps[0] += S.pe[jj] * out[sidx(cols, 0, jj)];
     red.template sum<1>(cl, ps);
     if (lead) {
       out[0] = (dg0 * fw[0] + ps[0]) / dg0;
@@ -994,8 +1027,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
         r[b] = on ? S.res[k] : 0.0;
         a[b] = on ? S.as[k] : 0.0;
         d[b] = on ? S.rdg[k] : 0.0;
-        // off-grid slots hold zeros; the row weight of any slot is finite
-        wr[b] = on ? S.rows[1 + pos_row(Rp, (int)(k % (unsigned)Rp))].s : 1.0;
+        wr[b] = on ? S.wt[k] : 0.0;
       }
 #pragma unroll
       for (int b = 0; b < kB; ++b) {
@@ -1004,7 +1036,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
         const double m = r[b] - alpha * a[b];
         S.mid[k] = m;
         S.pin[k] = m * d[b];
-        const double wv = m / wr[b];
+        const double wv = m * wr[b];
         d3[0] += wv * wv;
       }
     }
@@ -1065,7 +1097,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
         m[b] = on ? S.mid[k] : 0.0;
         a[b] = on ? S.am[k] : 0.0;
         h[b] = on ? S.shd[k] : 0.0;
-        wr[b] = on ? S.rows[1 + pos_row(Rp, (int)(k % (unsigned)Rp))].s : 1.0;
+        wr[b] = on ? S.wt[k] : 0.0;
       }
 #pragma unroll
       for (int b = 0; b < kB; ++b) {
@@ -1074,7 +1106,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
         S.x[k] = x[b] + (alpha * p[b] + omega * q[b]);
         const double r = m[b] - omega * a[b];
         S.res[k] = r;
-        const double wv = r / wr[b];
+        const double wv = r * wr[b];
         d5[0] += wv * wv;
         d5[1] += h[b] * r;
       }
@@ -1109,7 +1141,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
   // expand (nonorthogonal_mi.c:1130-1139); low-latitude potential is 0
   for (unsigned q = g; q < nq; q += G) {
     const int row = (int)(q / (unsigned)np), j = (int)(q - (unsigned)row * np);
-    S.pot[(size_t)(row + 1) * np + j] = S.x[sidx(Rp, row, j)];
+    S.pot[(size_t)(row + 1) * np + j] = S.x[sidx(cols, row, j)];
   }
   const double x0 = S.x[0];
   for (unsigned j = g; j < (unsigned)np; j += G) {
@@ -1156,70 +1188,12 @@ bool valid_tensor_config(const gamera_mi_solver_config *c) {
          c->longitude_count <= SIZE_MAX / c->colatitude_count;
 }
 
-using TensorKernel = void (*)(TSys);
-
-// Kernel instance of M chains per lane (1..8 or 16) and the group size.
-struct Launch {
-  TensorKernel kernel = nullptr;
-  int kRG = 0, G = 0;
-};
-
-Launch launch_for(int M, int G) {
-  if (G == 12) {
-    switch (M) {
-      case 1: return {k_tensor<1, 3, 12>, 3, 12};
-      case 2: return {k_tensor<2, 3, 12>, 3, 12};
-      case 3: return {k_tensor<3, 3, 12>, 3, 12};
-      case 4: return {k_tensor<4, 3, 12>, 3, 12};
-      case 5: return {k_tensor<5, 3, 12>, 3, 12};
-      case 6: return {k_tensor<6, 3, 12>, 3, 12};
-      default: return {};
-    }
-  }
-  if (G == 8) {
-    switch (M) {
-      case 1: return {k_tensor<1, 3, 8>, 3, 8};
-      case 2: return {k_tensor<2, 3, 8>, 3, 8};
-      case 3: return {k_tensor<3, 3, 8>, 3, 8};
-      case 4: return {k_tensor<4, 3, 8>, 3, 8};
-      case 5: return {k_tensor<5, 3, 8>, 3, 8};
-      case 6: return {k_tensor<6, 3, 8>, 3, 8};
-      case 7: return {k_tensor<7, 3, 8>, 3, 8};
-      case 8: return {k_tensor<8, 3, 8>, 3, 8};
-      default: return {};
-    }
-  }
-  if (G == 4) {
-    switch (M) {
-      case 1: return {k_tensor<1, 4, 4>, 4, 4};
-      case 2: return {k_tensor<2, 4, 4>, 4, 4};
-      case 3: return {k_tensor<3, 4, 4>, 4, 4};
-      case 4: return {k_tensor<4, 4, 4>, 4, 4};
-      case 5: return {k_tensor<5, 4, 4>, 4, 4};
-      case 6: return {k_tensor<6, 4, 4>, 4, 4};
-      case 7: return {k_tensor<7, 4, 4>, 4, 4};
-      case 8: return {k_tensor<8, 4, 4>, 4, 4};
-      case 16: return {k_tensor<16, 2, 4>, 2, 4};
-      default: return {};
-    }
-  }
-  switch (M) {
-    case 1: return {k_tensor<1, 16, 1>, 16, 1};
-    case 2: return {k_tensor<2, 16, 1>, 16, 1};
-    case 4: return {k_tensor<4, 16, 1>, 16, 1};
-    case 8: return {k_tensor<8, 16, 1>, 16, 1};
-    case 16: return {k_tensor<16, 8, 1>, 8, 1};
-    default: return {};
-  }
-}
-
 }  // namespace
 
 // Device buffers of one grid size, reused across calls.
 struct gcs_mi_tensor_plan {
   gamera_mi_solver_config config{};
   int np = 0, nt = 0, csize = 1;
-  TensorKernel kernel = nullptr;
   void *pool = nullptr;
   TSys sys{};
   double *d_fac = nullptr, *d_sp = nullptr, *d_sh = nullptr, *d_pot = nullptr;
@@ -1251,36 +1225,36 @@ cudaLaunchConfig_t launch_config(int csize, size_t smem, cudaStream_t stream,
   return cfg;
 }
 
-// Largest cluster (16, 8, 4, 2, 1 CTAs) the device can co-schedule.  The
-// kernel's shared-memory limit is set for the widest grid it serves, so a
-// plan for a narrower grid never lowers it under an earlier plan's need.
-int pick_cluster(const Launch &L, int Rp, size_t smem) {
-  size_t most = tensor_smem(L.kRG, L.G, Rp, kMaxLongitudes);
-  if (most > kSmemCap) most = kSmemCap;
-  if (cudaFuncSetAttribute(L.kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most) !=
-      cudaSuccess) {
+// Largest cluster (16, 8, 4, 2, 1 CTAs) the device can co-schedule, and its
+// shared memory; 0 if none.
+int pick_cluster(int blocks, int np, size_t *smem) {
+  // the limit is set once to the most any grid uses
+  if (cudaFuncSetAttribute(k_tensor, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)kSmemCap) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
-  if (cudaFuncSetAttribute(L.kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+  if (cudaFuncSetAttribute(k_tensor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
       cudaSuccess)
     cudaGetLastError();
   for (int c = kMaxCluster; c >= 1; c >>= 1) {
+    *smem = tensor_smem((blocks + c - 1) / c, np);
+    if (*smem > kSmemCap) continue;
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = launch_config(c, smem, nullptr, attr);
+    cudaLaunchConfig_t cfg = launch_config(c, *smem, nullptr, attr);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, L.kernel, &cfg) == cudaSuccess && n >= 1) return c;
+    if (cudaOccupancyMaxActiveClusters(&n, k_tensor, &cfg) == cudaSuccess && n >= 1) return c;
     cudaGetLastError();
   }
   return 0;
 }
 
 // True when one cluster of csize CTAs with smem bytes each can run.
-bool cluster_fits(TensorKernel k, int csize, size_t smem) {
+bool cluster_fits(int csize, size_t smem) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(csize, smem, nullptr, attr);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1) return true;
+  if (cudaOccupancyMaxActiveClusters(&n, k_tensor, &cfg) == cudaSuccess && n >= 1) return true;
   cudaGetLastError();
   return false;
 }
@@ -1295,21 +1269,14 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   gcs_mi_tensor_plan *p = new gcs_mi_tensor_plan();
   p->config = *c;
   const int np = (int)c->longitude_count, nt = (int)c->colatitude_count, R = nt - 2;
-  // sweep chains per lane: M = 1..8 or 16 with groups of 4 diagonals, which
-  // need the seam np - 1 >= 8 steps after the edge; narrower grids sweep one
-  // diagonal per group with M in {1, 2, 4, 8, 16}
-  const bool g4 = np >= 9;
-  int M = R <= 256 ? (R + 31) / 32 : 16;
-  if (!g4) M = M <= 1 ? 1 : M <= 2 ? 2 : M <= 4 ? 4 : M <= 8 ? 8 : 16;
-  const int Rp = 32 * M;  // rows of a diagonal
-  const int nrows = nt > Rp + 2 ? nt : Rp + 2;  // row table incl. padding rows
+  const int blocks = (R + kBlockRows - 1) / kBlockRows;
   p->np = np;
   p->nt = nt;
   const size_t nodes = (size_t)np * nt;
-  const size_t cols = 2 * (size_t)kPad + Rp + np - 1, len = cols * Rp;
-  // 12 vectors, 6 coefficient arrays and 2 coefficient pairs, all skewed
-  const size_t doubles = 4 * nodes + (12 + 6 + 4) * len + np + 2;
-  const size_t bytes = doubles * sizeof(double) + nrows * sizeof(TRow) +
+  const size_t cols = 2 * (size_t)kPad + np + 31, len = (size_t)blocks * cols * kBlockRows;
+  // 13 vectors, 6 coefficient arrays, 2 coefficient pairs and the index table
+  const size_t doubles = 4 * nodes + (13 + 6 + 4) * len + (len + 1) / 2 + np + 2;
+  const size_t bytes = doubles * sizeof(double) + nt * sizeof(TRow) +
                        sizeof(gamera_mi_solver_stats) + 64;
   if (!cuda_ok(cudaMalloc(&p->pool, bytes), "cudaMalloc") ||
       !cuda_ok(cudaMemset(p->pool, 0, bytes), "cudaMemset")) {
@@ -1323,13 +1290,14 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
     return r;
   };
   TSys &S = p->sys;
-  // skewed arrays first: len is a multiple of 32, so every diagonal the bulk
-  // copies touch starts on a 256-byte boundary
+  // skewed arrays first: len is a multiple of 64, so every column starts on a
+  // 512-byte boundary, as the sweeps' 16-byte copies and stores need
   S.cf = (double2 *)take(2 * len);
   S.cb = (double2 *)take(2 * len);
   double **vecs[] = {&S.rhs, &S.x, &S.res, &S.shd, &S.srch, &S.as, &S.psv, &S.mid,
-                     &S.pm, &S.am, &S.fw, &S.pin, &S.dg, &S.lo, &S.up, &S.ll, &S.lu, &S.rdg};
+                     &S.pm, &S.am, &S.fw, &S.pin, &S.wt, &S.dg, &S.lo, &S.up, &S.ll, &S.lu, &S.rdg};
   for (double **v : vecs) *v = take(len);
+  S.loc = (unsigned *)take((len + 1) / 2);
   p->d_fac = take(nodes);
   p->d_sp = take(nodes);
   p->d_sh = take(nodes);
@@ -1337,18 +1305,17 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   S.pe = take(np);
   S.pole_sum = take(2);
   TRow *rows = (TRow *)q;
-  S.stats = (gamera_mi_solver_stats *)(rows + nrows);
+  S.stats = (gamera_mi_solver_stats *)(rows + nt);
   S.status = (int *)(S.stats + 1);
   S.fault = S.status + 1;
   const double dth = c->maximum_colatitude / (double)(nt - 1);
-  // padding rows carry a unit row weight and nothing else
-  std::vector<TRow> hr(nrows, TRow{1.0, 0.0, 0.0, 0.0, 0.0, 0.0});
+  std::vector<TRow> hr(nt);
   for (int i = 0; i < nt; ++i) {
     const double th = (double)i * dth, lth = th - 0.5 * dth, uth = th + 0.5 * dth;
     hr[i] = TRow{sin(th), sin(lth), inc2(lth), sin(uth), inc2(uth),
                  cos_inclination(th, c->hemisphere)};
   }
-  if (!cuda_ok(cudaMemcpy(rows, hr.data(), nrows * sizeof(TRow), cudaMemcpyHostToDevice),
+  if (!cuda_ok(cudaMemcpy(rows, hr.data(), nt * sizeof(TRow), cudaMemcpyHostToDevice),
                "cudaMemcpy")) {
     plan_free(p);
     return nullptr;
@@ -1356,10 +1323,11 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   S.np = np;
   S.nt = nt;
   S.R = R;
-  S.Rp = Rp;
+  S.blocks = blocks;
+  S.cols = (int)cols;
   S.max_iter = c->maximum_iterations;
-  S.core0 = (unsigned)(kPad * (size_t)Rp);
-  S.core1 = (unsigned)((kPad + (size_t)Rp + np - 1) * Rp);
+  S.core0 = (unsigned)(kPad * kBlockRows);
+  S.core1 = (unsigned)(len - kPad * kBlockRows);
   S.dth = dth;
   S.dph = 2.0 * acos(-1.0) / (double)np;
   S.neg_r2 = -(c->ionosphere_radius_m * c->ionosphere_radius_m);
@@ -1376,16 +1344,7 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   S.sp = p->d_sp;
   S.sh = p->d_sh;
   S.pot = p->d_pot;
-  // (groups of 16 diagonals in a 2-slot ring were tried: 181 x 361 took
-  // 470 ms against 192 ms, each group waiting for its whole copy)
-  const int G = !g4 ? 1
-                : np >= 25 && M <= 6 && tensor_smem(3, 12, Rp, np) <= kSmemCap ? 12
-                : np >= 17 && M <= 8 && tensor_smem(3, 8, Rp, np) <= kSmemCap  ? 8
-                                                                                 : 4;
-  const Launch L = launch_for(M, G);
-  p->kernel = L.kernel;
-  p->smem = tensor_smem(L.kRG, L.G, Rp, np);
-  p->csize = L.kernel ? pick_cluster(L, Rp, p->smem) : 0;
+  p->csize = pick_cluster(blocks, np, &p->smem);
   if (p->csize == 0) {
     set_api_error("no thread-block cluster shape for the MI tensor solve");
     plan_free(p);
@@ -1401,7 +1360,7 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   if (p->csize >= 2) {
     const int h = (R + p->csize - 1) / p->csize;
     const size_t need = std::max(p->smem, band_smem(h, np));
-    if (h <= 32 && need <= kSmemCap && cluster_fits(p->kernel, p->csize, need)) {
+    if (h <= 32 && need <= kSmemCap && cluster_fits(p->csize, need)) {
       p->smem = need;
       p->band = h;
       p->nbands = (R + h - 1) / h;
@@ -1486,7 +1445,7 @@ int gcs_mi_tensor_solve_async(gcs_mi_tensor_plan *plan, void *stream) {
   if (!plan) return -1;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(plan->csize, plan->smem, (cudaStream_t)stream, attr);
-  return cuda_ok(cudaLaunchKernelEx(&cfg, plan->kernel, plan->sys), "MI tensor solve launch")
+  return cuda_ok(cudaLaunchKernelEx(&cfg, k_tensor, plan->sys), "MI tensor solve launch")
              ? 0
              : -1;
 }
