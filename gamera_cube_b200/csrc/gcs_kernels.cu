@@ -212,6 +212,48 @@ __global__ void k_halo_faces(Dims D, const HaloFace *plan, long long count,
   S.Po[dir][x] = of;
 }
 
+// CFL time-step reduction over active cells (nonorthogonal_step.c:449-525)
+// from the stored state; the driver loop's steps reduce it in k_update.
+__global__ void __launch_bounds__(256, 4) k_timestep(Dims D, DevState S, DevGeom G, DevBg BG,
+                                                 Opts O, DevStatus *st) {
+  // No early return: every thread reaches the block reduction below.
+  const bool skip = failed(st);
+  int f, i, j, k;
+  const Box b{D.g, D.g, D.g, D.n, D.n, D.g + D.nr};
+  double cand = DBL_MAX;
+  if (!skip && box_coord(b, &f, &i, &j, &k)) {
+    const long long c = f * D.Nn + D.node(i, j, k);
+    double u[5], bn[3], b0[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int m = 0; m < 5; ++m) u[m] = S.U[m][c];
+#pragma unroll
+    for (int m = 0; m < 3; ++m) {
+      bn[m] = S.B[m][c];
+      if (O.t_mhd && O.t_bg) b0[m] = BG.b0[m][c];
+    }
+    if (!cfl_step(O, u, bn, b0, G.cflmin[c], &cand)) fail(st, kStageTimestep, 0, f, i, j, k);
+  }
+  reduce_cfl(cand, st);
+}
+
+// Driver-mode time step (test_cubedsphere_dipole_background.c:593-670):
+// dt = min(fraction * cfl_min, 1.25 dt_prev), ratio = 0.5 dt / dt_prev
+// (0 on the first step).  Resets the reduction for the next step.
+__global__ void k_next_dt(StepParams *prm, DevStatus *st, double fraction) {
+  // the step just taken
+  const double prev = prm->dt;
+  prm->time += prev;
+  const int step = ++prm->step;
+  const double local = __longlong_as_double((long long)st->cfl_min_bits);
+  prm->cfl_min = local;
+  double dt = fraction * local;
+  if (step > 0) dt = fmin(dt, 1.25 * prev);
+  prm->ratio = step > 0 ? 0.5 * dt / prev : 0.0;
+  prm->dt_prev = prev;
+  prm->dt = dt;
+  st->cfl_min_bits = (unsigned long long)__double_as_longlong(DBL_MAX);
+}
+
 // ---------------------------------------------------------------------------
 // Host-side launchers.
 
