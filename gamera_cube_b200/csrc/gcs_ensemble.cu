@@ -340,10 +340,11 @@ gcs_ensemble *gcs_ensemble_create(const gcs_ensemble_config *cfg) {
       E->prev[i] = p;
     }
     E->runs[i] = ctx;
-    // one graph node per face or edge family: the branches of the step graph
-    // fill the GPU between them, and the node count of the graph stays what
-    // gcs_ensemble_graph_info has reported
-    ctx->c.X.split_families = 1;
+    // the short kernels keep a graph node per family, time level and counter,
+    // more than twenty a run, as gcs_ensemble_graph_info has reported; other
+    // branches of the graph run beside them.  The flux and EMF sweeps, where
+    // the families share cells in L2, run them in one launch
+    ctx->c.X.fine_launches = 1;
     if (rc != 0) {
       char msg[300];
       snprintf(msg, sizeof(msg), "run %d: %s", i, ctx->c.error);

@@ -24,7 +24,8 @@ namespace gcs {
 // Seam Phi synchronisation (cubedsphere_interface.c:7-38).  One thread per
 // seam face; each seam face belongs to exactly one (face, edge) pair.  The
 // seam flux synchronisation is k_seam_flux (gcs_sweeps.cuh).
-__global__ void k_seam_sync(Dims D, const Seam *seams, DevState S, DevStatus *st) {
+__global__ void k_seam_sync(Dims D, const Seam *seams, DevState S, int levels,
+                            DevStatus *st) {
   if (failed(st)) return;
   const long long per = (long long)D.nr * D.n;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
@@ -41,15 +42,15 @@ __global__ void k_seam_sync(Dims D, const Seam *seams, DevState S, DevStatus *st
   const long long s = sm.face * D.Nn + D.node(src[0], src[1], src[2]);
   const long long d = sm.nface * D.Nn + D.node(tgt[0], tgt[1], tgt[2]);
   const double o = sm.orient;
-  double *a = S.P[sm.src_axis], *b = S.P[sm.dst_axis];
-  double common = 0.5 * (a[s] + o * b[d]);
-  a[s] = common;
-  b[d] = o * common;
-  a = S.Po[sm.src_axis];
-  b = S.Po[sm.dst_axis];
-  common = 0.5 * (a[s] + o * b[d]);
-  a[s] = common;
-  b[d] = o * common;
+#pragma unroll
+  for (int l = 0; l < 2; ++l) {
+    if (!(levels >> l & 1)) continue;
+    double *a = l == 0 ? S.P[sm.src_axis] : S.Po[sm.src_axis];
+    double *b = l == 0 ? S.P[sm.dst_axis] : S.Po[sm.dst_axis];
+    const double common = 0.5 * (a[s] + o * b[d]);
+    a[s] = common;
+    b[d] = o * common;
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -239,11 +240,15 @@ __global__ void __launch_bounds__(256, 4) k_timestep(Dims D, DevState S, DevGeom
 // Driver-mode time step (test_cubedsphere_dipole_background.c:593-670):
 // dt = min(fraction * cfl_min, 1.25 dt_prev), ratio = 0.5 dt / dt_prev
 // (0 on the first step).  Resets the reduction for the next step.
-__global__ void k_next_dt(StepParams *prm, DevStatus *st, double fraction) {
-  // the step just taken
+// parts: bit 0 counts the step just taken, bit 1 sets the next one's size.
+__global__ void k_next_dt(StepParams *prm, DevStatus *st, double fraction, int parts) {
   const double prev = prm->dt;
-  prm->time += prev;
-  const int step = ++prm->step;
+  int step = prm->step;
+  if (parts & 1) {
+    prm->time += prev;
+    prm->step = ++step;
+  }
+  if (!(parts & 2)) return;
   const double local = __longlong_as_double((long long)st->cfl_min_bits);
   prm->cfl_min = local;
   double dt = fraction * local;
@@ -302,10 +307,11 @@ Bulk<double> bulk64(const Ctx &X) {
 
 void launch_seam_sync(const Ctx &X, int magnetic, cudaStream_t s) {
   const long long total = 12LL * X.D.nr * X.D.n;
-  if (magnetic)
-    k_seam_sync<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(X.D, X.seams, X.S,
-                                                                X.status);
-  else
+  if (magnetic) {
+    for (int l = X.fine_launches ? 1 : 3; l <= (X.fine_launches ? 2 : 3); ++l)
+      k_seam_sync<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(X.D, X.seams, X.S, l,
+                                                                  X.status);
+  } else
     k_seam_flux<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(X.D, X.seams, X.S,
                                                                 X.status);
 }
@@ -381,7 +387,7 @@ void launch_edge_sync(const Ctx &X, cudaStream_t s) {
 void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s) {
   const Dims &D = X.D;
   const Tile t = X.tile[kTileCt], tu = X.tile[kTileUpdate];
-  for (int d = X.split_families ? 0 : -1; d < (X.split_families ? 3 : 0); ++d)
+  for (int d = X.fine_launches ? 0 : -1; d < (X.fine_launches ? 3 : 0); ++d)
     k_ct<<<tile_grid(D.E0 + 1, D.E1 + 1, D.E2 + 1, t), tile_block(t), 0, s>>>(
         D, X.S, O, d < 0 ? 7 : 1 << d, X.params, X.status);
   if (O.u_mhd) launch_seam_sync(X, 1, s);
@@ -405,7 +411,8 @@ void launch_set_failure(const Ctx &X, int stage, int dir, cudaStream_t s) {
 }
 
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s) {
-  k_next_dt<<<1, 1, 0, s>>>(X.params, X.status, fraction);
+  for (int parts = X.fine_launches ? 1 : 3; parts <= (X.fine_launches ? 2 : 3); ++parts)
+    k_next_dt<<<1, 1, 0, s>>>(X.params, X.status, fraction, parts);
 }
 
 // Whole step in reference order.

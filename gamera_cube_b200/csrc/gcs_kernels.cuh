@@ -40,7 +40,9 @@ struct Ctx {
   StepParams *params = nullptr;   // device
   DevStatus *status = nullptr;    // device
   int ortho = 0;                  // 1: every active face frame is orthonormal
-  int split_families = 0;         // 1: a launch per face or edge family (ensembles)
+  // 1: the short kernels (face velocities, CT, the Phi sync, the step counter)
+  // with a launch per family, time level or counter (ensembles)
+  int fine_launches = 0;
   int flux_staged = 0;            // 1: TMA-staged flux sweeps (gcs_flux_tma.cuh)
   int bulk = 0;                   // 1: FP32-bulk sweeps (B32)
   int bulk_split = 0;             // radial layers [0, bulk_split) stay FP64

@@ -550,23 +550,6 @@ inline dim3 boxes_grid(const Boxes &X, int groups, Tile t) {
   for (int q = 0; q < 3; ++q) points = max(points, X.b[q].nj * X.b[q].nk);
   return dim3((unsigned)((points + t.bx - 1) / t.bx), 3u * (unsigned)groups, kFaces);
 }
-// A sweep's launches over [i0, i1): all families at once, or one at a time
-// (Ctx::split_families).
-template <typename Launch>
-void launch_families(const Ctx &X, Boxes b, const int lo[3], const int hi[3], int i0, int i1,
-                     Tile t, Launch launch) {
-  for (int only = X.split_families ? 0 : -1; only < (X.split_families ? 3 : 0); ++only) {
-    int l[3], h[3];
-    for (int q = 0; q < 3; ++q) {
-      const bool on = only < 0 || q == only;
-      l[q] = on ? lo[q] : 0;
-      h[q] = on ? hi[q] : 0;
-    }
-    const int groups = clamp_boxes(b, l, h, i0, i1, t);
-    if (groups > 0) launch(boxes_grid(b, groups, t), b);
-  }
-}
-
 template <typename T>
 struct Sweeps {
   static void flux(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
@@ -589,10 +572,10 @@ struct Sweeps {
     const int lo[3] = {D.g, D.g, D.g}, hi[3] = {D.g + D.nr + 1, D.g + D.nr, D.g + D.nr};
     // FP32 reads the tangents: its rounded frame is not orthonormal to FP32
     const bool ortho = X.ortho && sizeof(T) == 8;
-    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
+    const int groups = clamp_boxes(b, lo, hi, i0, i1, t);
+    if (groups > 0)
       (ortho ? k_flux<true, T> : k_flux<false, T>)
-          <<<grid, tile_block(t), 0, s>>>(D, X.S, B, O, X.status, boxes);
-    });
+          <<<boxes_grid(b, groups, t), tile_block(t), 0, s>>>(D, X.S, B, O, X.status, b);
   }
   static void emf(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                   cudaStream_t s) {
@@ -611,9 +594,19 @@ struct Sweeps {
       hi[a] = first[0] + count[0];
       b.b[a] = Box{0, first[1], first[2], count[1], count[2], 0};
     }
-    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
-      k_face_velocity<T><<<grid, tile_block(t), 0, s>>>(D, B, X.status, boxes);
-    });
+    // all families at once, or one at a time (Ctx::fine_launches)
+    for (int only = X.fine_launches ? 0 : -1; only < (X.fine_launches ? 3 : 0); ++only) {
+      int l[3], h[3];
+      for (int a = 0; a < 3; ++a) {
+        const bool on = only < 0 || a == only;
+        l[a] = on ? lo[a] : 0;
+        h[a] = on ? hi[a] : 0;
+      }
+      const int groups = clamp_boxes(b, l, h, i0, i1, t);
+      if (groups > 0)
+        k_face_velocity<T><<<boxes_grid(b, groups, t), tile_block(t), 0, s>>>(D, B, X.status,
+                                                                              b);
+    }
   }
   static void edge(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                    cudaStream_t s) {
@@ -626,10 +619,10 @@ struct Sweeps {
       hi[e] = D.g + D.nr + (e != 0);
       b.b[e] = Box{0, D.g, D.g, D.n + (e != 1), D.n + (e != 2), 0};
     }
-    launch_families(X, b, lo, hi, i0, i1, t, [&](dim3 grid, const Boxes &boxes) {
-      k_edge_emf<T><<<grid, tile_block(t), 0, s>>>(D, X.S, X.G, B, O, X.params, X.status,
-                                                   boxes);
-    });
+    const int groups = clamp_boxes(b, lo, hi, i0, i1, t);
+    if (groups > 0)
+      k_edge_emf<T><<<boxes_grid(b, groups, t), tile_block(t), 0, s>>>(
+          D, X.S, X.G, B, O, X.params, X.status, b);
   }
 };
 
