@@ -30,6 +30,12 @@
 // Bound: the chain of a step (a shuffle and two dependent fused
 // multiply-adds).  Two rows per lane make np + R / 2 steps of the chain where
 // one row per lane would make np + R with a chain one multiply-add shorter.
+// Measured at 361 x 181 (449 iterations): one warp sweeping whole
+// anti-diagonals 167-175 ms, this 93 ms.  A group of eight steps takes some 1,010
+// to 1,230 cycles: 730 for the steps, 230 for issuing the copies ahead, 150
+// for taking the neighbouring block's row.  Slower: the copies and operand
+// loads spread between the steps (105 ms), groups of four (115), a second
+// warp that copies (112).
 //
 // Band schedule (the default on grids narrower than 17 longitudes): the
 // same sweeps with the rows split into one band per CTA, each band swept by
@@ -63,10 +69,9 @@ using gcs::set_api_error;
 namespace {
 
 // Sweep blocks of 64 rows (two per lane), up to 8 of them.  A sweep warp
-// works in groups of kGroup steps and prefetches its operands up to 24 steps
-// ahead into a ring of kRing: an L2 round trip of some 700 cycles is about 12
-// steps.
-constexpr int kRing = 32;
+// prefetches its operands kRing steps deep (32, or 16 where many sweep warps
+// share a CTA) in groups of 8 steps: the ring covers an L2 round trip of some
+// 700 cycles at about 50 cycles a step.
 constexpr int kThreads = 256;
 constexpr int kMaxRows = 512;
 constexpr int kBlockRows = 64;
@@ -235,6 +240,10 @@ __device__ __forceinline__ double inbox_peek(const double *p) {
   return v;
 }
 
+__device__ __forceinline__ bool is_empty(double v) {
+  return __double2hiint(v) == (int)(kEmpty >> 32);
+}
+
 // Value of an inbox slot, waiting (bounded) for it to arrive; false when
 // it never did.
 __device__ __forceinline__ bool inbox_take(const double *p, double &v) {
@@ -260,102 +269,66 @@ __host__ __device__ constexpr int inbox_len(int np) { return np + 2 * kInboxPad 
 
 // Shared memory of the sweep warps of one CTA: per warp a prefetch ring and
 // the two inboxes (the row below the block for the forward sweep, above it
-// for the reverse).  Block 0 receives no row below: the pole edges by column
-// (zero off the grid) are kept in its place.
+// for the reverse), and the pole edges by column (CTA 0; zero off the grid).
 struct WaveMem {
   unsigned char *ring;    // [warps][kRing][kStepBytes]
   double *inf, *inr;      // [warps][inbox_len]
-  double *pe;             // [inbox_len], CTA 0
+  double *pe;             // [inbox_len]
 };
 
-// What a sweep warp holds between steps.
+// What a sweep warp holds between groups.
 struct WaveState {
   double v0, v1;          // the lane's two rows at the previous step
   double edge0, edge1;    // ... at the sweep's first longitude
   double seam0, seam1;    // seam coefficients of the two rows
   double psum;
 };
-// A step's operands of the lane: two values, two coefficient pairs.
-struct WaveOperands {
-  double2 a, c0, c1;
-  __device__ __forceinline__ void load(const unsigned char *at) {
-    a = *reinterpret_cast<const double2 *>(at);
-    c0 = *reinterpret_cast<const double2 *>(at + 512);
-    c1 = *reinterpret_cast<const double2 *>(at + 1024);
-  }
-};
-// Where the copies of a group's steps come from and go to.
-struct WaveCopy {
-  const double *a;
-  const double2 *c;
-  unsigned to;
-};
-constexpr int kEmptyHigh = (int)(kEmpty >> 32);
 
-// The kGroup steps of one group; col0 is the first step's column, vo and
-// to_next its output and neighbour inbox addresses.  kEdgy: the group holds a
-// point on the first or last longitude; kPole: block 0 of the reverse sweep.
-//
-// A step is a chain of some 50 cycles (a shuffle, a select and two
-// multiply-adds) with few instructions of its own, so everything else is
-// placed between the steps: the operands of four steps on are loaded from the
-// ring (o[u % 4]), those of 24 steps on are copied into it, and halfway
-// through the linking lane looks at the neighbouring block's row of the next
-// group (next_e).
+// The kGroup steps of one group, operands already in the ring at `at`; col0
+// is the first step's column, dir = +-1 the direction, vo and to_next the
+// first step's output and neighbour inbox addresses.  kEdgy: the group holds
+// a point on the first or last longitude; kPole: block 0 of the reverse sweep.
+// All operands are loaded before the first step, so a step is the shuffle,
+// four multiply-adds and two stores.
 template <bool kReverse, bool kEdgy, bool kPole>
-__device__ __forceinline__ void wave_group(WaveState &s, WaveOperands (&o)[4],
-                                           const unsigned char *here,
-                                           const unsigned char *there, const WaveCopy &cp,
-                                           bool copying, const double (&e)[kGroup],
-                                           double (&next_e)[kGroup], const double *next_in,
-                                           bool linked, bool link, unsigned send, int col0,
-                                           int np, double *vo, unsigned to_next,
+__device__ __forceinline__ void wave_group(WaveState &s, const unsigned char *at,
+                                           const double (&e)[kGroup], bool link, bool send,
+                                           int col0, int np, double *vo, unsigned to_next,
                                            const double *pe) {
   constexpr int dir = kReverse ? -1 : 1;
   const int lane = threadIdx.x & 31;
+  double2 a[kGroup], c0[kGroup], c1[kGroup];
+#pragma unroll
+  for (int u = 0; u < kGroup; ++u) {
+    a[u] = *reinterpret_cast<const double2 *>(at + u * kStepBytes);
+    c0[u] = *reinterpret_cast<const double2 *>(at + u * kStepBytes + 512);
+    c1[u] = *reinterpret_cast<const double2 *>(at + u * kStepBytes + 1024);
+  }
 #pragma unroll
   for (int u = 0; u < kGroup; ++u) {
     const int j = col0 + dir * u - lane;
-    double t0 = o[u % 4].a.x, t1 = o[u % 4].a.y;
     if (kEdgy && j == (kReverse ? 0 : np - 1)) {
-      t0 = fma(-s.seam0, s.edge0, t0);
-      t1 = fma(-s.seam1, s.edge1, t1);
+      a[u].x = fma(-s.seam0, s.edge0, a[u].x);
+      a[u].y = fma(-s.seam1, s.edge1, a[u].y);
     }
     double x = kReverse ? __shfl_down_sync(0xffffffffu, s.v0, 1)
                         : __shfl_up_sync(0xffffffffu, s.v1, 1);
-    t0 = fma(-o[u % 4].c0.y, s.v0, t0);
-    t1 = fma(-o[u % 4].c1.y, s.v1, t1);
-    const double c0x = o[u % 4].c0.x, c1x = o[u % 4].c1.x;
-    o[u % 4].load((u + 4 < kGroup ? here : there) + ((u + 4) % kGroup) * kStepBytes);
-    if (copying) {
-      copy16(cp.to + u * kStepBytes, cp.a + dir * u * kBlockRows);
-      copy16(cp.to + u * kStepBytes + 512, cp.c + dir * u * kBlockRows);
-      copy16(cp.to + u * kStepBytes + 1024, cp.c + dir * u * kBlockRows + 32);
-    }
     x = link ? e[u] : x;
+    const double t0 = fma(-c0[u].y, s.v0, a[u].x), t1 = fma(-c1[u].y, s.v1, a[u].y);
     if (kReverse) {
-      s.v1 = fma(-c1x, x, t1);
-      s.v0 = fma(-c0x, s.v1, t0);
+      s.v1 = fma(-c1[u].x, x, t1);
+      s.v0 = fma(-c0[u].x, s.v1, t0);
     } else {
-      s.v0 = fma(-c0x, x, t0);
-      s.v1 = fma(-c1x, s.v0, t1);
+      s.v0 = fma(-c0[u].x, x, t0);
+      s.v1 = fma(-c1[u].x, s.v0, t1);
     }
     if (kEdgy && j == (kReverse ? np - 1 : 0)) {
       s.edge0 = s.v0;
       s.edge1 = s.v1;
     }
-    // (predicated, not branched around: one lane sends)
-    asm volatile(
-        "{\n .reg .pred p;\n setp.ne.u32 p, %2, 0;\n"
-        " @p st.relaxed.cluster.shared::cluster.b64 [%0], %1;\n}" ::"r"(
-            to_next + (unsigned)(dir * u * 8)),
-        "d"(kReverse ? s.v0 : s.v1), "r"(send));
+    if (send) inbox_put(to_next + (unsigned)(dir * u * 8), kReverse ? s.v0 : s.v1);
     *reinterpret_cast<double2 *>(vo + dir * u * kBlockRows) = make_double2(s.v0, s.v1);
     if (kPole) s.psum = fma(pe[dir * u], s.v0, s.psum);
-    if (linked && u == kGroup / 2) {
-#pragma unroll
-      for (int q = 0; q < kGroup; ++q) next_e[q] = inbox_peek(next_in + dir * q);
-    }
   }
 }
 
@@ -366,26 +339,39 @@ __device__ __forceinline__ void wave_group(WaveState &s, WaveOperands (&o)[4],
 // (nonorthogonal_mi.c:910-964); off-grid points read zeros and produce zeros.
 // psum accumulates the pole edge sum over row 0 (block 0).  Returns false
 // when a value of the neighbouring block never arrived: the fault is recorded
-// and the remaining steps use what the inbox holds.
-template <bool kReverse>
-__device__ __noinline__ bool wave_sweep(const TSys &S, const double *__restrict__ in,
-                                        double *__restrict__ out, const WaveMem &wm,
-                                        int slot, int w, int csize, double boundary,
-                                        double &psum) {
-  // groups copied beyond the current one; the next one has landed when a
-  // group begins
-  constexpr int kAhead = kRing / kGroup - 1;
-  static_assert(kAhead >= 2, "the ring holds the current, the next and a copied group");
+// and the remaining steps use zeros.
+// kLinked: the grid has more than one block.
+template <int kRing, bool kReverse, bool kLinked>
+__device__ __forceinline__ bool wave_sweep(const TSys &S, const double *__restrict__ in,
+                                           double *__restrict__ out, const WaveMem &wm,
+                                           int slot, int w, int csize, double boundary,
+                                           double &psum) {
+  constexpr int kAhead = kRing / kGroup - 1;  // groups in flight beyond the current one
   constexpr int dir = kReverse ? -1 : 1;
   const int lane = threadIdx.x & 31, np = S.np;
   const int ngroups = (np + 31 + kGroup - 1) / kGroup;
   const int start = kReverse ? np + 30 : 0;   // first column
   const size_t base = ((size_t)w * S.cols + kPad + start) * kBlockRows;
-  WaveCopy cp{in + base + 2 * lane, (kReverse ? S.cb : S.cf) + base + lane, 0u};
+  const double *va = in + base + 2 * lane;
+  const double2 *co = (kReverse ? S.cb : S.cf) + base + lane;
   double *vo = out + base + 2 * lane;
   unsigned char *ring = wm.ring + (size_t)slot * kRing * kStepBytes + lane * 16;
   const unsigned ring_at = smem_u32(ring);
-  auto slot_of = [&](int g) { return (unsigned)((g * kGroup) & (kRing - 1)) * (unsigned)kStepBytes; };
+  // the operands of the next group (steps past the last read padding zeros)
+  unsigned next_slot = 0u;
+  auto issue = [&]() {
+    const unsigned at = ring_at + next_slot;
+#pragma unroll
+    for (int u = 0; u < kGroup; ++u) {
+      copy16(at + u * kStepBytes, va + dir * u * kBlockRows);
+      copy16(at + u * kStepBytes + 512, co + dir * u * kBlockRows);
+      copy16(at + u * kStepBytes + 1024, co + dir * u * kBlockRows + 32);
+    }
+    va += dir * kGroup * kBlockRows;
+    co += dir * kGroup * kBlockRows;
+    next_slot += kGroup * kStepBytes;
+    if (next_slot == kRing * kStepBytes) next_slot = 0u;
+  };
   WaveState s{};
   {
     // the other sweep's pair at this sweep's last longitude
@@ -395,9 +381,10 @@ __device__ __noinline__ bool wave_sweep(const TSys &S, const double *__restrict_
     s.seam0 = sc[0].y;
     s.seam1 = sc[32].y;
   }
-  const bool from = kReverse ? w + 1 < S.blocks : w > 0;
+  const bool from = kLinked && (kReverse ? w + 1 < S.blocks : w > 0);
   const bool link = kReverse ? lane == 31 : lane == 0;
-  const bool send = kReverse ? lane == 0 && w > 0 : lane == 31 && w + 1 < S.blocks;
+  const bool send =
+      kLinked && (kReverse ? lane == 0 && w > 0 : lane == 31 && w + 1 < S.blocks);
   double *boxes = kReverse ? wm.inr : wm.inf;
   double *inbox = boxes + (size_t)slot * inbox_len(np) + kInboxPad;  // by longitude
   unsigned to_next = 0u;   // the sending lane's longitude is its column less its lane
@@ -410,81 +397,47 @@ __device__ __noinline__ bool wave_sweep(const TSys &S, const double *__restrict_
   const double *pe = wm.pe + kInboxPad + start;
   const double fixed = kReverse ? 0.0 : boundary;
   bool ok = true;
-  auto copy_group = [&]() {
-#pragma unroll
-    for (int u = 0; u < kGroup; ++u) {
-      copy16(cp.to + u * kStepBytes, cp.a + dir * u * kBlockRows);
-      copy16(cp.to + u * kStepBytes + 512, cp.c + dir * u * kBlockRows);
-      copy16(cp.to + u * kStepBytes + 1024, cp.c + dir * u * kBlockRows + 32);
-    }
-  };
-  auto next_copy = [&]() {
-    cp.a += dir * kGroup * kBlockRows;
-    cp.c += dir * kGroup * kBlockRows;
-  };
 #pragma unroll
   for (int g = 0; g < kAhead; ++g) {
-    if (g < ngroups) {
-      cp.to = ring_at + slot_of(g);
-      copy_group();
-      next_copy();
-    }
+    if (g < ngroups) issue();
     asm volatile("cp.async.commit_group;" ::: "memory");
   }
-  asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
-  WaveOperands o[4];
-#pragma unroll
-  for (int u = 0; u < 4; ++u) o[u].load(ring + u * kStepBytes);
-  // the linking lane's first longitude of group k in the neighbour's row
-  auto row_at = [&](int k) { return start + dir * k * kGroup - (kReverse ? 31 : 0); };
-  double e[kGroup], next_e[kGroup];
-#pragma unroll
-  for (int u = 0; u < kGroup; ++u)
-    next_e[u] = from ? __longlong_as_double((long long)kEmpty) : fixed;
   for (int k = 0; k < ngroups; ++k) {
     const int col0 = start + dir * k * kGroup;
+    asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 1) : "memory");
+    if (k + kAhead < ngroups) issue();
+    asm volatile("cp.async.commit_group;" ::: "memory");
+    double e[kGroup];
 #pragma unroll
-    for (int u = 0; u < kGroup; ++u) e[u] = next_e[u];
-    // the next group's operands have landed too
-    asm volatile("cp.async.wait_group %0;" ::"n"(kAhead - 2) : "memory");
+    for (int u = 0; u < kGroup; ++u) e[u] = fixed;
     if (from) {
-      const int j0 = row_at(k);
-      // longitudes off the grid are not waited for (their points are zero)
-      auto missing = [&]() {
-        bool any = false;
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u)
-          any = any || (__double2hiint(e[u]) == kEmptyHigh &&
-                        (unsigned)(j0 + dir * u) < (unsigned)np);
-        return any && link;
-      };
-      unsigned tries = 0;
-      while (__any_sync(0xffffffffu, missing()) && ok) {
-#pragma unroll
-        for (int u = 0; u < kGroup; ++u) e[u] = inbox_peek(inbox + j0 + dir * u);
+      // the neighbouring block's row at this group's longitudes, one to a lane
+      const double *row = inbox + col0 + dir * (lane & (kGroup - 1)) - (kReverse ? 31 : 0);
+      double x = inbox_peek(row);
+      // (the whole warp polls: lanes leaving a loop one by one cost the first
+      // group of every following block some 4,000 cycles)
+      for (unsigned tries = 0; ok && __any_sync(0xffffffffu, is_empty(x));) {
+        x = inbox_peek(row);
         ok = ++tries < kInboxSpinLimit;
       }
+      // the linking lane reads what the lanes above have seen arrive
+      __syncwarp();
 #pragma unroll
       for (int u = 0; u < kGroup; ++u)
-        if (__double2hiint(e[u]) == kEmptyHigh) e[u] = 0.0;
+        e[u] = ok ? inbox_peek(inbox + col0 + dir * u - (kReverse ? 31 : 0)) : 0.0;
     }
-    const unsigned char *here = ring + slot_of(k), *there = ring + slot_of(k + 1);
-    cp.to = ring_at + slot_of(k + kAhead);
-    const bool copying = k + kAhead < ngroups, linked = from && k + 1 < ngroups;
-    const double *next_in = inbox + row_at(k + 1);
+    const unsigned char *at =
+        ring + (size_t)((k * kGroup) & (kRing - 1)) * kStepBytes;
     // the only groups with a point on the first or the last longitude
     const int last = col0 + dir * (kGroup - 1);
-    if (pole)
-      wave_group<kReverse, true, true>(s, o, here, there, cp, copying, e, next_e, next_in,
-                                       linked, link, send, col0, np, vo, to_next, pe);
-    else if (min(col0, last) <= 31 || max(col0, last) >= np - 1)
-      wave_group<kReverse, true, false>(s, o, here, there, cp, copying, e, next_e, next_in,
-                                        linked, link, send, col0, np, vo, to_next, pe);
-    else
-      wave_group<kReverse, false, false>(s, o, here, there, cp, copying, e, next_e, next_in,
-                                         linked, link, send, col0, np, vo, to_next, pe);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    next_copy();
+    const bool edgy = min(col0, last) <= 31 || max(col0, last) >= np - 1;
+    if (pole) {
+      wave_group<kReverse, true, true>(s, at, e, link, send, col0, np, vo, to_next, pe);
+    } else if (edgy) {
+      wave_group<kReverse, true, false>(s, at, e, link, send, col0, np, vo, to_next, pe);
+    } else {
+      wave_group<kReverse, false, false>(s, at, e, link, send, col0, np, vo, to_next, pe);
+    }
     vo += dir * kGroup * kBlockRows;
     to_next += (unsigned)(dir * kGroup * 8);
     pe += dir * kGroup;
@@ -610,11 +563,13 @@ __device__ __forceinline__ bool locate(const TSys &S, unsigned k, int &row, int 
 }
 
 // Dynamic shared memory of a launch: the rings and inboxes of the CTA's
-// sweep warps.
-size_t tensor_smem(int warps, int np) {
-  return (size_t)warps * (kRing * kStepBytes + 2 * inbox_len(np) * sizeof(double));
+// sweep warps and the pole-edge table.
+size_t tensor_smem(int ring, int warps, int np) {
+  return (size_t)warps * ring * kStepBytes +
+         (size_t)(2 * warps + 1) * inbox_len(np) * sizeof(double);
 }
 
+template <int kRing>
 __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
   constexpr int kT = kThreads, kWarps = kT / 32;
   constexpr int kB = 5;  // grid points a thread loads per batch
@@ -633,7 +588,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
   wm.ring = reinterpret_cast<unsigned char *>(dyn_smem);
   wm.inf = dyn_smem + (size_t)sweepers * kRing * (kStepBytes / sizeof(double));
   wm.inr = wm.inf + (size_t)sweepers * inbox_len(np);
-  wm.pe = wm.inf;
+  wm.pe = wm.inr + (size_t)sweepers * inbox_len(np);
   // the band schedule's tables share the dynamic shared memory
   BandMem bm;
   bm.h = S.band;
@@ -647,10 +602,13 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     bm.pe = bm.inr + np;
   }
   {
+    // an inbox's slots off the grid are never empty: nothing waits for them
     double *inboxes = S.band ? bm.inf : wm.inf;
     const int n = 2 * (S.band ? np : sweepers * inbox_len(np));
-    for (int j = threadIdx.x; j < n; j += kT)
-      inboxes[j] = __longlong_as_double((long long)kEmpty);
+    for (int j = threadIdx.x; j < n; j += kT) {
+      const bool on = S.band != 0 || (unsigned)(j % inbox_len(np) - kInboxPad) < (unsigned)np;
+      inboxes[j] = on ? __longlong_as_double((long long)kEmpty) : 0.0;
+    }
   }
   if (rank == 0 && t == 0) *S.fault = 0;
   const unsigned g = (unsigned)(rank * kT + t), G = (unsigned)(csize * kT);
@@ -860,9 +818,14 @@ __global__ void __launch_bounds__(kThreads, 1) k_tensor(TSys S) {
     const int w = rank + warp * csize;
     const double in0 = w == 0 ? in[0] : 0.0;
     double psum = 0.0;
-    if (wave_sweep<false>(S, in, S.fw, wm, warp, w, csize, in0, psum) &&
-        wave_sweep<true>(S, S.fw, out, wm, warp, w, csize, 0.0, psum) && w == 0 &&
-        lane == 0) {
+    bool done;
+    if (S.blocks > 1)
+      done = wave_sweep<kRing, false, true>(S, in, S.fw, wm, warp, w, csize, in0, psum) &&
+             wave_sweep<kRing, true, true>(S, S.fw, out, wm, warp, w, csize, 0.0, psum);
+    else
+      done = wave_sweep<kRing, false, false>(S, in, S.fw, wm, warp, w, csize, in0, psum) &&
+             wave_sweep<kRing, true, false>(S, S.fw, out, wm, warp, w, csize, 0.0, psum);
+    if (done && w == 0 && lane == 0) {
       // pole (nonorthogonal_mi.c:958-963): (dg0 fw0 + sum pe_j out(1, j)) / dg0
       out[0] = (dg0 * in0 + psum) / dg0;
       *S.pole_sum = psum;
@@ -1188,12 +1151,15 @@ bool valid_tensor_config(const gamera_mi_solver_config *c) {
          c->longitude_count <= SIZE_MAX / c->colatitude_count;
 }
 
+using TensorKernel = void (*)(TSys);
+
 }  // namespace
 
 // Device buffers of one grid size, reused across calls.
 struct gcs_mi_tensor_plan {
   gamera_mi_solver_config config{};
   int np = 0, nt = 0, csize = 1;
+  TensorKernel kernel = nullptr;
   void *pool = nullptr;
   TSys sys{};
   double *d_fac = nullptr, *d_sp = nullptr, *d_sh = nullptr, *d_pot = nullptr;
@@ -1225,36 +1191,45 @@ cudaLaunchConfig_t launch_config(int csize, size_t smem, cudaStream_t stream,
   return cfg;
 }
 
-// Largest cluster (16, 8, 4, 2, 1 CTAs) the device can co-schedule, and its
-// shared memory; 0 if none.
-int pick_cluster(int blocks, int np, size_t *smem) {
-  // the limit is set once to the most any grid uses
-  if (cudaFuncSetAttribute(k_tensor, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kSmemCap) != cudaSuccess) {
-    cudaGetLastError();
-    return 0;
-  }
-  if (cudaFuncSetAttribute(k_tensor, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
-      cudaSuccess)
-    cudaGetLastError();
+// Kernel and shared memory for clusters of csize CTAs: the deep ring where the
+// CTA's sweep warps leave room for it.
+size_t launch_for(int csize, int blocks, int np, TensorKernel *kernel) {
+  const int warps = (blocks + csize - 1) / csize;
+  const size_t deep = tensor_smem(32, warps, np);
+  *kernel = deep <= kSmemCap ? k_tensor<32> : k_tensor<16>;
+  return deep <= kSmemCap ? deep : tensor_smem(16, warps, np);
+}
+
+// Largest cluster (16, 8, 4, 2, 1 CTAs) the device can co-schedule, its kernel
+// and shared memory; 0 if none.
+int pick_cluster(int blocks, int np, TensorKernel *kernel, size_t *smem) {
   for (int c = kMaxCluster; c >= 1; c >>= 1) {
-    *smem = tensor_smem((blocks + c - 1) / c, np);
+    *smem = launch_for(c, blocks, np, kernel);
     if (*smem > kSmemCap) continue;
+    // the limit is set once to the most any grid uses
+    if (cudaFuncSetAttribute(*kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)kSmemCap) != cudaSuccess) {
+      cudaGetLastError();
+      return 0;
+    }
+    if (cudaFuncSetAttribute(*kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+        cudaSuccess)
+      cudaGetLastError();
     cudaLaunchAttribute attr[1];
     cudaLaunchConfig_t cfg = launch_config(c, *smem, nullptr, attr);
     int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k_tensor, &cfg) == cudaSuccess && n >= 1) return c;
+    if (cudaOccupancyMaxActiveClusters(&n, *kernel, &cfg) == cudaSuccess && n >= 1) return c;
     cudaGetLastError();
   }
   return 0;
 }
 
 // True when one cluster of csize CTAs with smem bytes each can run.
-bool cluster_fits(int csize, size_t smem) {
+bool cluster_fits(TensorKernel k, int csize, size_t smem) {
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(csize, smem, nullptr, attr);
   int n = 0;
-  if (cudaOccupancyMaxActiveClusters(&n, k_tensor, &cfg) == cudaSuccess && n >= 1) return true;
+  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) == cudaSuccess && n >= 1) return true;
   cudaGetLastError();
   return false;
 }
@@ -1344,7 +1319,7 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   S.sp = p->d_sp;
   S.sh = p->d_sh;
   S.pot = p->d_pot;
-  p->csize = pick_cluster(blocks, np, &p->smem);
+  p->csize = pick_cluster(blocks, np, &p->kernel, &p->smem);
   if (p->csize == 0) {
     set_api_error("no thread-block cluster shape for the MI tensor solve");
     plan_free(p);
@@ -1360,7 +1335,7 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
   if (p->csize >= 2) {
     const int h = (R + p->csize - 1) / p->csize;
     const size_t need = std::max(p->smem, band_smem(h, np));
-    if (h <= 32 && need <= kSmemCap && cluster_fits(p->csize, need)) {
+    if (h <= 32 && need <= kSmemCap && cluster_fits(p->kernel, p->csize, need)) {
       p->smem = need;
       p->band = h;
       p->nbands = (R + h - 1) / h;
@@ -1445,7 +1420,7 @@ int gcs_mi_tensor_solve_async(gcs_mi_tensor_plan *plan, void *stream) {
   if (!plan) return -1;
   cudaLaunchAttribute attr[1];
   cudaLaunchConfig_t cfg = launch_config(plan->csize, plan->smem, (cudaStream_t)stream, attr);
-  return cuda_ok(cudaLaunchKernelEx(&cfg, k_tensor, plan->sys), "MI tensor solve launch")
+  return cuda_ok(cudaLaunchKernelEx(&cfg, plan->kernel, plan->sys), "MI tensor solve launch")
              ? 0
              : -1;
 }
