@@ -11,12 +11,11 @@
 //
 // One thread-block cluster solves one system and keeps it on chip for the
 // whole solve.  CTA c of the cluster owns a contiguous band of colatitude
-// rows; the search direction lives in the CTA's shared memory (neighbours
-// read the adjacent row of the band through distributed shared memory), the
-// solution and residual live in registers, and every dot product is a
-// block reduction followed by one cluster barrier and a fixed-order sum of
-// the CTAs' partials, so all CTAs see bit-identical scalars and take the
-// same branches.  Several systems (the two hemispheres) are independent
+// rows; what the neighbours in the grid read lives in the CTA's shared memory
+// (edge rows cross between CTAs through distributed shared memory), the other
+// vectors live in registers, and a reduction is a block reduction followed by
+// one cluster barrier and a fixed-order sum of the CTAs' partials, so all
+// CTAs see bit-identical scalars and take the same branches.  Several systems (the two hemispheres) are independent
 // clusters of one launch.  HBM is touched only to load the inputs and store
 // the potential.
 #include <cooperative_groups.h>

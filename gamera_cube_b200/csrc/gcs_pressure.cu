@@ -46,7 +46,7 @@ __device__ inline unsigned long long warp_max(unsigned long long v) {
 }
 
 // CFL candidate of one active cell (nonorthogonal_step.c:449-525, the same
-// arithmetic as the recovery kernel's fused CFL reduction): false when the
+// arithmetic as the update kernel's fused CFL reduction): false when the
 // reference fails the cell.
 __device__ inline bool cfl_candidate(const double u[5], const double bn[3], const double *b0,
                                      double cflmin, const Opts &O, double *cand) {

@@ -15,26 +15,6 @@
 // sweep launch covers one radial range [i0, i1).
 #pragma once
 
-#ifndef GCS_F32_FLUX_BLOCKS
-#define GCS_F32_FLUX_BLOCKS 6
-#endif
-#ifndef GCS_F32_EDGE_BLOCKS
-#define GCS_F32_EDGE_BLOCKS 8
-#endif
-#ifndef GCS_PREDICT_BLOCKS
-#define GCS_PREDICT_BLOCKS 4
-#endif
-#ifndef GCS_UPDATE_BLOCKS
-#define GCS_UPDATE_BLOCKS 4
-#endif
-#ifndef GCS_FLUX_BLOCKS
-#define GCS_FLUX_BLOCKS 4
-#endif
-#ifndef GCS_EDGE_BLOCKS
-#define GCS_EDGE_BLOCKS 6
-#endif
-
-
 #include "gcs_kernel_util.cuh"
 #include "gcs_kernels.cuh"
 #include "gcs_physics.cuh"
@@ -50,7 +30,7 @@ namespace gcs {
 // B~ in FP64; primitives of U~ with the sweep options (rho NaN where the
 // conversion fails), Phi~/area and the EMF weights V m / max(rho, floor)
 // for the sweeps, in FP64 and (bulk) FP32.
-__global__ void __launch_bounds__(256, GCS_PREDICT_BLOCKS) k_predict(Dims D, DevState S, DevGeom G, Bulk<float> B32, int bulk,
+__global__ void __launch_bounds__(256, 4) k_predict(Dims D, DevState S, DevGeom G, Bulk<float> B32, int bulk,
                           Opts O, const StepParams *prm, DevStatus *st) {
   const unsigned long long first = failure_word(st);
   int f, i, j, k;
@@ -138,17 +118,17 @@ __global__ void __launch_bounds__(256, GCS_PREDICT_BLOCKS) k_predict(Dims D, Dev
 #endif  // GCS_SWEEPS_TEMPLATES_ONLY
 
 // Minimum resident blocks of 128 threads per SM the sweeps are compiled for
-// (register caps 128 and 96 in FP64, 64 in FP32), from measured full-step
+// (register caps 128 and 80 in FP64, 80 and 64 in FP32), from measured full-step
 // sweeps at 6 x 96x96x192.
 template <typename T>
 struct SweepOccupancy {
-  static constexpr int flux = GCS_FLUX_BLOCKS;
-  static constexpr int edge = GCS_EDGE_BLOCKS;
+  static constexpr int flux = 4;
+  static constexpr int edge = 6;
 };
 template <>
 struct SweepOccupancy<float> {
-  static constexpr int flux = GCS_F32_FLUX_BLOCKS;
-  static constexpr int edge = GCS_F32_EDGE_BLOCKS;
+  static constexpr int flux = 6;
+  static constexpr int edge = 8;
 };
 
 // ---------------------------------------------------------------------------
@@ -422,7 +402,7 @@ __global__ void k_ct(Dims D, DevState S, Opts O, int families, const StepParams 
 // SM (124 registers): at six, the bound without the recovery, it spills.
 // 6 x 96x96x192, CT, update and recovery: 2.72 -> 1.79 ms a step (six blocks
 // 2.21, five 1.99).
-__global__ void __launch_bounds__(128, GCS_UPDATE_BLOCKS) k_update(Dims D, DevState S, DevGeom G,
+__global__ void __launch_bounds__(128, 4) k_update(Dims D, DevState S, DevGeom G,
                                                 DevBg BG, Opts O, int with_cfl,
                                                 const StepParams *prm,
                                                 DevStatus *st) {

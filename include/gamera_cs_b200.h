@@ -148,9 +148,8 @@ int gamera_mi_solve_constant_pedersen(const gamera_mi_solver_config *config,
 int gamera_mi_apply_conductance_tensor(const gamera_mi_solver_config *config,
                                        const double *pedersen, const double *hall,
                                        const double *potential_v, double *result);
-/* nonorthogonal_mi.h:99-102.  SSOR-BiCGStab on one GPU CTA: the SSOR
- * sweeps run as row wavefronts with the reference's per-point arithmetic;
- * at most 512 interior colatitude rows. */
+/* nonorthogonal_mi.h:99-102.  SSOR-BiCGStab on one thread-block
+ * cluster: the SSOR sweeps run as wavefronts, a warp to 64 rows; at most 512 interior colatitude rows. */
 int gamera_mi_solve_conductance_tensor(const gamera_mi_solver_config *config,
                                        const double *fac_a_m2, const double *pedersen,
                                        const double *hall, double *potential_v,
