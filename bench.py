@@ -45,24 +45,29 @@ METRIC = "MHD cell-updates/s on 1 B200 (FP64 plain path)"
 # Algorithmic bytes per cell-update of the whole step (state 192 B +
 # compacted metric 664 B + background 192 B).
 STEP_BYTES_PER_CELL = 1048
-# Per-launch algorithmic bytes per face of the flux sweep: cells U~ (5),
-# B~ (3), volume (1) counted once per face along the sweep, face Phi~ (1),
-# area (1), frame (9), central8 volume (1), B0 face (3) + B0 normal (1),
-# written fluid (5) + Maxwell (3) flux: 33 doubles.
-FLUX_BYTES_PER_FACE = 33 * 8
-# Edge EMF per edge: face velocities (3) and areas (1) of one face family,
-# Phi~ (2) and areas (1) of the other, edge frame (6), 2x2 system (5),
-# central8 area sums (2), length (1), B0 projections (2), edge density
-# cells (1), written EMF (1): 25 doubles (each counted once per edge).
+# Kernels of a step graph: seam Phi sync, cell halos, radial outflow, face
+# halos, predictor, flux, seam flux sync, face velocities, edge EMF, edge sync,
+# CT, seam Phi sync, update, next time step.
+STEP_KERNELS = 14
+# Algorithmic bytes per face of the flux sweep (one launch for the three face
+# families, orthonormal frames): cells U~ (5), B~ (3), volume (1) counted once
+# per cell, a third per face; face Phi~ (1), area (1), normal (3), central8
+# volume (1), B0 face (3) + B0 normal (1), written fluid (5) + Maxwell (3)
+# flux: 21 doubles.
+FLUX_BYTES_PER_FACE = 21 * 8
+# Edge EMF per edge (one launch for the three edge families): face velocities
+# (3) and areas (1) of one face family, Phi~ (2) and areas (1) of the other,
+# edge frame (6), 2x2 system (5), central8 area sums (2), length (1), B0
+# projections (2), edge density cells (1), written EMF (1): 25 doubles (each
+# counted once per edge).
 EMF_BYTES_PER_EDGE = 25 * 8
-# Measured DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) per
-# face of a flux launch and per edge of an edge-EMF launch: the mean of the
-# three launches of each sweep in an ncu capture of the 6 x 32x32x48 case
-# (state arrays larger than L2), divided by the faces or edges one launch
-# processes there.  The sweeps stream their arrays, so the traffic of a
-# launch of the bench's workload is these figures times its faces or edges.
-FLUX_TRAFFIC_BYTES_PER_FACE = 310.6
-EMF_TRAFFIC_BYTES_PER_EDGE = 277.7
+# Measured DRAM bytes (dram__bytes_read.sum + dram__bytes_write.sum) of a flux
+# and an edge-EMF launch in an ncu capture of the 6 x 48x48x64 case (state
+# arrays larger than L2), divided by the faces or edges of the launch.  The
+# sweeps stream their arrays, so the traffic of a launch of the bench's
+# workload is these figures times its faces or edges.
+FLUX_TRAFFIC_BYTES_PER_FACE = 194.4
+EMF_TRAFFIC_BYTES_PER_EDGE = 225.6
 
 
 def peaks():
@@ -284,13 +289,11 @@ def run_gpu(args):
         alg = cells * STEP_BYTES_PER_CELL
     traffic = None
     if dom == "flux":
-        traffic = faces_per_dir * FLUX_TRAFFIC_BYTES_PER_FACE
+        traffic = 3 * faces_per_dir * FLUX_TRAFFIC_BYTES_PER_FACE
     elif dom == "edge_emf":
-        traffic = edges_per_dir * EMF_TRAFFIC_BYTES_PER_EDGE
-    per_launch_ms = stages[dom] / 3.0 if dom in ("flux", "edge_emf") else stages[dom]
+        traffic = 3 * edges_per_dir * EMF_TRAFFIC_BYTES_PER_EDGE
     hbm, peak_kind = peaks()
-    achieved = (alg / 3.0 if dom in ("flux", "edge_emf") else alg) / (
-        per_launch_ms * 1e-3) / 1e9
+    achieved = alg / (stages[dom] * 1e-3) / 1e9
 
     # ---- end to end through the drop-in step with pinned host buffers
     act = (C.c_size_t * 3)()
@@ -352,7 +355,7 @@ def run_gpu(args):
     result = None
     if rank == 0:
         clk = clocks.summary()
-        launches_per_step = 24 + (7 if had_mi else 0)
+        launches_per_step = STEP_KERNELS + (7 if had_mi else 0)
         result = {
             "metric": METRIC,
             "value": value,
@@ -379,7 +382,7 @@ def run_gpu(args):
                        "parallelism": "replicas x%d" % world,
                        "setup_s": round(setup_s, 2)},
             "gpu_launches": launches_per_step * args.steps,
-            "gpu_launches_note": "24 kernels per step graph + 7 of the ionosphere "
+            "gpu_launches_note": "14 kernels per step graph + 7 of the ionosphere "
                                  "coupling in every step's graph (cadence, 4 FAC "
                                  "kernels, 1 two-hemisphere solve, check), which "
                                  "return at once on steps where the update is not "
@@ -405,10 +408,9 @@ def run_gpu(args):
                          if peak_kind == "measured" else "fallback 6650 GB/s",
                          "traffic": traffic,
                          "traffic_source": None if traffic is None else
-                         "ncu DRAM bytes per launch of a 6x32x32x48 capture, scaled "
+                         "ncu DRAM bytes per launch of a 6x48x48x64 capture, scaled "
                          "by faces/edges per launch",
-                         "algorithmic_bytes_per_launch": alg / 3.0
-                         if dom in ("flux", "edge_emf") else alg,
+                         "algorithmic_bytes_per_launch": alg,
                          "step_share": stages[dom] / step_ms_prof,
                          "step_hbm_frac": cells * STEP_BYTES_PER_CELL /
                          (ms_local / args.steps * 1e-3) / 1e9 / hbm},
@@ -601,13 +603,13 @@ def run_earth(lib, torch, device, args, dist, ctx):
                         "constant upstream monitor" % (act[1], act[2], act[0]),
             "call": "gcs_context_run_earth (device driver loop, one CUDA graph per step)",
             "boundary_device_bytes": nbytes,
-            "gpu_launches_per_step": 24 + 18,
+            "gpu_launches_per_step": STEP_KERNELS + 18,
             "with_pressure_control": {
                 "ms_per_step": ms_pc / args.earth_steps,
                 "arguments": "gamma 5/3, floors 1e-6/1e-8, c 10, low density 1e-3, "
                              "low-density sound speed 1e-7",
                 "low_density_cells": pc_low.value, "high_sound_speed_cells": pc_hot.value,
-                "gpu_launches_per_step": 24 + 18 + 1,
+                "gpu_launches_per_step": STEP_KERNELS + 18 + 1,
                 "active": {
                     "ms_per_step": ms_pca / args.earth_steps,
                     "arguments": "gamma 5/3, floors 1e-6/1e-8, thresholds from the state: "
@@ -841,12 +843,12 @@ def run_mi(lib, torch, device, solves):
         "e2e_call": "gamera_mi_solve_constant_pedersen (drop-in, host arrays, "
                     "H2D/D2H of %d B each way)" % (2 * nodes * 8),
         "effective_gbs": eff,
-        "bound": "latency (2 cluster barriers per iteration; vectors on chip)",
+        "bound": "latency (1 cluster barrier per iteration; vectors on chip)",
         "solves_timed": solves,
         "tensor": {"operator": "Pedersen + Hall (1.5x) tensor, SSOR-BiCGStab",
                    "ms_per_call": tensor_ms,
                    "iterations": tensor_its,
-                   "launch": "one thread-block cluster (16 CTAs); SSOR sweeps by one warp along anti-diagonals, diagonals moved by bulk async copies",
+                   "launch": "one thread-block cluster (16 CTAs); SSOR sweeps by a warp per 64 rows along anti-diagonals, operands prefetched by async copies",
                    "colored_ordering": {"ms_per_call": colored_ms, "iterations": colored_its,
                                         "sweep": "four-colour SSOR, each colour by the whole cluster"}},
         "tensor_two_level": two_level,
