@@ -309,7 +309,7 @@ int run_step(gcs_context *ctx, const gcs::Opts &O, int driver_mode,
 
 void report_failure(gcs::Context &C) {
   const unsigned long long v = C.host_status.first;
-  const int stage = (int)(v >> 56) & 0xff;
+  const int stage = gcs::failure_stage(v);
   const char *rank = getenv("PMI_RANK");
   if (!rank) rank = getenv("SLURM_PROCID");
   fprintf(stderr,
@@ -1200,7 +1200,7 @@ int gcs_context_failure(gcs_context *ctx, int *dir, int *face, int *i, int *j,
   if (i) *i = (int)(v >> 32) & 0xffff;
   if (j) *j = (int)(v >> 16) & 0xffff;
   if (k) *k = (int)v & 0xffff;
-  return (int)(v >> 56) & 0xff;
+  return gcs::failure_stage(v);
 }
 
 int gcs_context_reset_failure(gcs_context *ctx) {

@@ -180,7 +180,7 @@ enum Stage : int {
 };
 
 struct DevStatus {
-  unsigned long long first;      // packed first failure (0 = none)
+  unsigned long long first;      // packed first failure (0 = none), kEarlierStep
   unsigned int stage_mask;       // bit per failed stage
   unsigned int pad;
   unsigned long long emergency_count[kFaces];
@@ -188,15 +188,53 @@ struct DevStatus {
   unsigned long long cfl_min_bits;                // min CFL step as bits
 };
 
+// Bit of DevStatus::first: the failure belongs to an earlier stage or step.
+constexpr unsigned long long kEarlierStep = 1ULL << 63;
+
+GCS_HD inline int failure_stage(unsigned long long first) { return (int)(first >> 56) & 0x7f; }
+
+// Position in the step of the stage group a failure belongs to.  Kernels of
+// one group may run side by side (the three directions of a sweep, its FP64
+// and FP32 layers); groups follow one another.
+enum StagePass {
+  kPassNone = 0, kPassPredict, kPassFlux, kPassEmf, kPassUpdate, kPassFinal, kPassTimestep,
+  kPassOther
+};
+
 GCS_HD inline unsigned long long pack_failure(int stage, int dir,
                                                           int face, int i,
                                                           int j, int k) {
-  return ((unsigned long long)(stage & 0xff) << 56) |
+  return ((unsigned long long)(stage & 0x7f) << 56) |
          ((unsigned long long)(dir & 0xf) << 52) |
          ((unsigned long long)(face & 0xf) << 48) |
          ((unsigned long long)(i & 0xffff) << 32) |
          ((unsigned long long)(j & 0xffff) << 16) |
          (unsigned long long)(k & 0xffff);
+}
+
+GCS_HD inline int stage_pass(int stage) {
+  switch (stage) {
+    case kStageNone: return kPassNone;
+    case kStagePredict: case kStageRecoverPredict: return kPassPredict;
+    case kStageReconstruct: case kStageKineticFluid: case kStageKineticMaxwell:
+    case kStageEmergency: case kStageTileCopy: return kPassFlux;
+    case kStageEdgeGeometry: case kStageEdgeVelocity: case kStageTransverse:
+    case kStageEdgeDensity: case kStageEdgeEmf: case kStageSolveEdge: return kPassEmf;
+    case kStageUpdate: case kStageRecoverUpdate: return kPassUpdate;
+    case kStageRecoverFinal: return kPassFinal;
+    case kStageTimestep: return kPassTimestep;
+    default: return kPassOther;
+  }
+}
+
+// Whether failure a is reported before failure b: the earlier stage group,
+// then the lower direction, face and indices, whichever thread met its own
+// first.
+GCS_HD inline bool fails_before(unsigned long long a, unsigned long long b) {
+  if (b & kEarlierStep) return false;
+  const int pa = stage_pass(failure_stage(a)), pb = stage_pass(failure_stage(b));
+  constexpr unsigned long long kWhere = (1ULL << 56) - 1;
+  return pa != pb ? pa < pb : (a & kWhere) < (b & kWhere);
 }
 
 // Halo plan entries (built on the host from the reference geometry).

@@ -126,7 +126,7 @@ __device__ __forceinline__ void face_flux(int d, const Stencil &cells, const Dim
       apply_hogs(&fl, &mx, st2, inv_gm1<T>(O), (T)O.hogs_h, (T)O.hogs_m, O.s_boris,
                  (T)O.s_ic2);
   }
-  if (first != 0ULL) return;
+  if (stopped(first, kPassFlux)) return;
   if (!(recon_ok && fluid_ok && maxwell_ok)) {
     fail(st, !recon_ok ? kStageReconstruct : !fluid_ok ? kStageKineticFluid
                                                        : kStageKineticMaxwell,

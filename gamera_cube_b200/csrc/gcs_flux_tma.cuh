@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256, FluxTile<d, T>::MIN_BLOCKS)
   // a block leaves before its first copy if an earlier kernel of the step
   // failed (one thread reads the status, so the whole block agrees)
   if (tid == 0) {
-    skip = failed(st) ? 1 : 0;
+    skip = stopped(failure_word(st), kPassFlux) ? 1 : 0;
     if (!skip) {
       for (int q = 0; q < Sh::STAGES; ++q) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(&full[q])));

@@ -13,7 +13,13 @@ namespace {
 
 __device__ inline void fail(DevStatus *st, int stage, int dir, int face,
                             int i, int j, int k) {
-  atomicCAS(&st->first, 0ULL, pack_failure(stage, dir, face, i, j, k));
+  const unsigned long long mine = pack_failure(stage, dir, face, i, j, k);
+  unsigned long long seen = atomicCAS(&st->first, 0ULL, mine);
+  while (seen != 0ULL && fails_before(mine, seen)) {
+    const unsigned long long was = atomicCAS(&st->first, seen, mine);
+    if (was == seen) break;
+    seen = was;
+  }
   atomicOr(&st->stage_mask, 1u << stage);
 }
 
@@ -25,6 +31,18 @@ __device__ inline unsigned long long failure_word(const DevStatus *st) {
   return *(volatile const unsigned long long *)&st->first;
 }
 __device__ inline bool failed(const DevStatus *st) { return failure_word(st) != 0ULL; }
+// Whether a kernel of stage groups [pass, last] has to leave everything as it
+// is: a failure of an earlier group or step.  A failure of its own groups
+// stops no thread, so the one reported, and what the others store, do not
+// depend on the order in which the blocks run.
+__device__ inline bool stopped(unsigned long long first, int pass, int last) {
+  if (first == 0ULL) return false;
+  const int p = stage_pass(failure_stage(first));
+  return (first & kEarlierStep) != 0ULL || p < pass || p > last;
+}
+__device__ inline bool stopped(unsigned long long first, int pass) {
+  return stopped(first, pass, pass);
+}
 
 // Box iteration over radial layers [i0, i1): a thread block is a tile of
 // blockDim.x consecutive points of the flattened (j, k) plane times

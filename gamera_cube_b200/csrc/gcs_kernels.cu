@@ -26,9 +26,13 @@ namespace gcs {
 // seam flux synchronisation is k_seam_flux (gcs_sweeps.cuh).
 __global__ void k_seam_sync(Dims D, const Seam *seams, DevState S, int levels,
                             DevStatus *st) {
-  if (failed(st)) return;
-  const long long per = (long long)D.nr * D.n;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (failed(st)) {
+    // the stages that follow belong to a later group or step
+    if (t == 0) atomicOr(&st->first, kEarlierStep);
+    return;
+  }
+  const long long per = (long long)D.nr * D.n;
   if (t >= 12 * per) return;
   const Seam sm = seams[t / per];
   const int rem = (int)(t % per);
@@ -218,7 +222,7 @@ __global__ void k_halo_faces(Dims D, const HaloFace *plan, long long count,
 __global__ void __launch_bounds__(256, 4) k_timestep(Dims D, DevState S, DevGeom G, DevBg BG,
                                                  Opts O, DevStatus *st) {
   // No early return: every thread reaches the block reduction below.
-  const bool skip = failed(st);
+  const bool skip = stopped(failure_word(st), kPassTimestep);
   int f, i, j, k;
   const Box b{D.g, D.g, D.g, D.n, D.n, D.g + D.nr};
   double cand = DBL_MAX;

@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256, 4) k_predict(Dims D, DevState S, DevGeom 
     prv[3] = pr.vz;
     prv[4] = pr.p;
   }
-  if (first != 0ULL) return;
+  if (stopped(first, kPassPredict)) return;
 #pragma unroll
   for (int d = 0; d < 3; ++d) {
     if (!in[d]) continue;
@@ -300,7 +300,7 @@ __device__ __forceinline__ void edge_thread(const Dims &D, const DevState &S,
   const bool emf_ok =
       edge_emf(vt1, vt2, ef0, ef1, jump, (T)rho, B.elen[e][cb], (T)O.e_diff, O.e_boris,
                (T)O.e_c, (T)(O.e_cfl * Num<double>::rcp(prm->dt)), &emf) == 0;
-  if (first != 0ULL) return;
+  if (stopped(first, kPassEmf)) return;
   if (geometry != 0 || !rho_ok || !emf_ok) {
     fail(st, geometry != 0 ? geometry : !rho_ok ? kStageEdgeDensity : kStageEdgeEmf, e, f,
          x[0], x[1], x[2]);
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(128, 4) k_update(Dims D, DevState S, DevGeom G
         }
       }
     }
-    if (first == 0ULL) {
+    if (!stopped(first, kPassUpdate, kPassTimestep)) {
 #pragma unroll
       for (int m = 0; m < 5; ++m) S.Uo[m][c] = uold[m];
 #pragma unroll

@@ -315,7 +315,9 @@ int gcs_context_params(gcs_context *ctx, double *dt, double *ratio,
                        double *cfl_min, int *steps);
 int gcs_context_set_params(gcs_context *ctx, double dt, double ratio,
                            double dt_prev, int steps);
-/* First failure since the last reset; returns the stage code (0 = none). */
+/* First failure since the last reset; returns the stage code (0 = none).
+ * Of failures in one stage group (predictor, flux sweeps, EMF sweeps,
+ * update) the lowest direction's, then the lowest face's and index's. */
 int gcs_context_failure(gcs_context *ctx, int *dir, int *face, int *i, int *j,
                         int *k);
 int gcs_context_reset_failure(gcs_context *ctx);
