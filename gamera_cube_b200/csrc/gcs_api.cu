@@ -321,6 +321,18 @@ void report_failure(gcs::Context &C) {
           (int)(v >> 16) & 0xffff, (int)v & 0xffff);
 }
 
+// Outcome of a step whose kernels are queued; after a failed update the state
+// has the B that the step began with.
+bool step_failed(gcs::Context &C) {
+  if (!device_failed(C)) return false;
+  if (gcs::update_failed(C.host_status.first)) {
+    gcs::launch_undo_magnetic(C.X, C.stream);
+    cudaStreamSynchronize(C.stream);
+  }
+  report_failure(C);
+  return true;
+}
+
 std::mutex g_registry_mutex;
 std::map<const void *, gcs_context *> g_registry;
 
@@ -424,8 +436,7 @@ int drop_in_step(gcs_context *ctx, const gamera_no_grid grid[6],
     const bool hooks = radial || options->fluid_flux_sync || options->edge_emf_sync;
     rc = run_step(ctx, O, 0, hooks ? &hk : nullptr);
   }
-  const bool fail = device_failed(C);
-  if (fail) report_failure(C);
+  const bool fail = step_failed(C);
   // Emergency-diffusion statistics accumulate in the caller's storage.
   for (int f = 0; f < 6; ++f) {
     storage[f].emergency_diffusion_face_count += C.host_status.emergency_count[f];
@@ -977,8 +988,7 @@ int gcs_context_step(gcs_context *ctx, const gamera_no_advance_options *options,
     return -1;
   C.reset_status_async();
   const int rc = run_step(ctx, O, 0, nullptr);
-  const bool fail = device_failed(C);
-  if (fail) report_failure(C);
+  const bool fail = step_failed(C);
   return (rc != 0 || fail) ? -1 : 0;
 }
 
@@ -1008,8 +1018,7 @@ int gcs_context_step_earth(gcs_context *ctx, gcs_earth *earth,
   // (test_cubedsphere_dipole_background.c:667-668)
   const gcs::EarthStep es{&earth->dev, current_time, previous_time, current_time, dt, 0};
   const int rc = run_step(ctx, O, 0, nullptr, &es);
-  const bool fail = device_failed(C);
-  if (fail) report_failure(C);
+  const bool fail = step_failed(C);
   return (rc != 0 || fail) ? -1 : 0;
 }
 

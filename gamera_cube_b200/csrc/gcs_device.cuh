@@ -227,6 +227,10 @@ GCS_HD inline int stage_pass(int stage) {
   }
 }
 
+GCS_HD inline bool update_failed(unsigned long long first) {
+  return stage_pass(failure_stage(first)) == kPassUpdate;
+}
+
 // Whether failure a is reported before failure b: the earlier stage group,
 // then the lower direction, face and indices, whichever thread met its own
 // first.

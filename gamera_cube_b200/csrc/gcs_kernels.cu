@@ -241,11 +241,34 @@ __global__ void __launch_bounds__(256, 4) k_timestep(Dims D, DevState S, DevGeom
   reduce_cfl(cand, st);
 }
 
+// k_update stores each cell's B with its U.  Where the update of a cell fails,
+// the step has stopped before the final recovery in the stage order, so the
+// other cells get back the B that the step began with, which k_update has
+// saved as B_old.
+__device__ inline void undo_magnetic(const Dims &D, const DevState &S, long long t,
+                                     long long threads) {
+  for (long long c = t; c < kFaces * D.Nn; c += threads)
+#pragma unroll
+    for (int m = 0; m < 3; ++m) S.B[m][c] = S.Bo[m][c];
+}
+__global__ void k_undo_magnetic(Dims D, DevState S) {
+  undo_magnetic(D, S, blockIdx.x * (long long)blockDim.x + threadIdx.x,
+                gridDim.x * (long long)blockDim.x);
+}
+
 // Driver-mode time step (test_cubedsphere_dipole_background.c:593-670):
 // dt = min(fraction * cfl_min, 1.25 dt_prev), ratio = 0.5 dt / dt_prev
 // (0 on the first step).  Resets the reduction for the next step.
 // parts: bit 0 counts the step just taken, bit 1 sets the next one's size.
-__global__ void k_next_dt(StepParams *prm, DevStatus *st, double fraction, int parts) {
+// One block: thread 0 sets the step, all undo a failed update's B.
+__global__ void __launch_bounds__(1024) k_next_dt(Dims D, DevState S, StepParams *prm,
+                                                  DevStatus *st, double fraction, int parts) {
+  if (parts & 2) {
+    const unsigned long long first = failure_word(st);
+    if (!(first & kEarlierStep) && update_failed(first))
+      undo_magnetic(D, S, threadIdx.x, blockDim.x);
+  }
+  if (threadIdx.x != 0) return;
   const double prev = prm->dt;
   int step = prm->step;
   if (parts & 1) {
@@ -416,7 +439,11 @@ void launch_set_failure(const Ctx &X, int stage, int dir, cudaStream_t s) {
 
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s) {
   for (int parts = X.fine_launches ? 1 : 3; parts <= (X.fine_launches ? 2 : 3); ++parts)
-    k_next_dt<<<1, 1, 0, s>>>(X.params, X.status, fraction, parts);
+    k_next_dt<<<1, 1024, 0, s>>>(X.D, X.S, X.params, X.status, fraction, parts);
+}
+
+void launch_undo_magnetic(const Ctx &X, cudaStream_t s) {
+  k_undo_magnetic<<<592, 256, 0, s>>>(X.D, X.S);
 }
 
 // Whole step in reference order.

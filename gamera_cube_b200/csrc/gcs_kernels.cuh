@@ -92,6 +92,9 @@ void launch_edge_sync(const Ctx &X, cudaStream_t s);
 // with_cfl: also the CFL reduction of the new state into status.
 void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s);
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s);
+// B of every cell as it was before the update that failed (driver mode:
+// launch_next_dt does it on the device).
+void launch_undo_magnetic(const Ctx &X, cudaStream_t s);
 void launch_step(const Ctx &X, const Opts &O, int driver_mode,
                  cudaStream_t s);
 // CFL reduction alone (nonorthogonal_step.c:449-525) into status.

@@ -11,7 +11,7 @@ from oracle import oracle_cases
 
 pytestmark = pytest.mark.gpu
 
-KINETIC_MAXWELL, EDGE_EMF = 5, 11
+KINETIC_MAXWELL, EDGE_EMF, UPDATE = 5, 11, 12
 
 
 @pytest.fixture(scope="module")
@@ -77,3 +77,43 @@ def test_first_failure_is_of_the_lowest_direction(lib, case, family):
             at[cell_] = value
     assert stage == (KINETIC_MAXWELL if family == "flux" else EDGE_EMF)
     assert (d, face, cell) == (0, 5, (g + nr - 1, g + n - 2, g + n - 1))
+
+
+@pytest.mark.parametrize("mode", ["drop_in", "step", "run", "run_graph"])
+def test_failed_update_leaves_the_field(lib, case, mode):
+    """A NaN background force fails the momentum update of one cell: the step
+    stops there, and B of every active cell is the one it began with."""
+    g, (nr, n) = case.ghost, list(case.active)[:2]
+    ext = [nr + 2 * g, n + 2 * g, n + 2 * g]
+    act = (slice(g, g + nr), slice(g, g + n), slice(g, g + n))
+    cell = (g + 3, g + 5, g + 7)
+    force = field(case.background[2].cell_force, ext)
+    kept = force[cell].copy()
+    before = [case.arrays(f)["cell_magnetic"][act].copy() for f in range(6)]
+    force[cell] = np.nan
+    try:
+        if mode == "drop_in":
+            stage, _, face, at = failed_step(lib, case)
+        else:
+            ctx = lib.gcs_context_create(case.grid, case.active, case.ghost)
+            assert ctx, lib.gcs_last_error()
+            assert lib.gcs_context_upload_background(ctx, case.background) == 0
+            assert lib.gcs_context_upload_state(ctx, case.storage) == 0
+            if mode == "step":
+                assert lib.gcs_context_step(ctx, case.options, 0.0,
+                                            0.4 * case.local_timestep()) == -1
+            else:
+                assert lib.gcs_context_run(ctx, case.options, case.timestep_options, 0.5, 3,
+                                           int(mode == "run_graph")) == 0
+                assert lib.gcs_context_sync(ctx) == -1
+            v = [C.c_int() for _ in range(5)]
+            stage = lib.gcs_context_failure(ctx, *[C.byref(q) for q in v])
+            face, at = v[1].value, tuple(q.value for q in v[2:])
+            assert lib.gcs_context_download_state(ctx, case.storage, 0) == 0
+            lib.gcs_context_destroy(ctx)
+    finally:
+        force[cell] = kept
+    assert (stage, face, at) == (UPDATE, 2, cell)
+    for f in range(6):
+        now = case.arrays(f)["cell_magnetic"][act]
+        np.testing.assert_array_equal(now, before[f])
