@@ -111,6 +111,7 @@ struct Context {
   int upload_background(const gamera_no_background_field bg[kFaces]);
   bool background_matches(const gamera_no_background_field bg[kFaces]) const;
   int transfer_array(int f, int kind, int dir, bool upload, double *host);
+  int member_staging();
   int move_state(const gamera_no_storage st[kFaces], bool upload);
   int upload_state(const gamera_no_storage st[kFaces]);
   int download_state(gamera_no_storage st[kFaces], int scratch);

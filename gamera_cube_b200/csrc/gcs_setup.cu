@@ -351,18 +351,19 @@ struct StateArrays {
   long long start[10], count[10];
 };
 
-// Staging to device arrays (upload) or back, one launch per face: a thread
-// per point and array.
+// Staging to device arrays (upload) or back, arrays first, first + 1, ... of
+// a face (one per blockIdx.y) from the start of `stage`: a thread per point
+// and array.
 template <bool kUpload>
-__global__ void k_move_state(Dims D, int f, StateArrays A, double *stage) {
-  const int a = blockIdx.y;
+__global__ void k_move_state(Dims D, int f, StateArrays A, int first, double *stage) {
+  const int a = first + blockIdx.y;
   const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (t >= A.count[a]) return;
   const int e1 = A.e[a][1], e2 = A.e[a][2];
   const int k = (int)(t % e2), j = (int)((t / e2) % e1), i = (int)(t / ((long long)e1 * e2));
   const long long c = f * D.Nn + D.node(i, j, k);
   const int n = A.comps[a];
-  double *s = stage + A.start[a] + t * n;
+  double *s = stage + (A.start[a] - A.start[first]) + t * n;
 #pragma unroll
   for (int q = 0; q < 5; ++q) {
     if (q >= n) break;
@@ -838,12 +839,7 @@ int Context::transfer_array(int f, int kind, int dir, bool upload, double *host)
   }
   const long long count = (long long)e[0] * e[1] * e[2];
   const size_t bytes = (size_t)count * ncomp * sizeof(double);
-  if (!staging && owner) {
-    // runs sharing a grid allocate their transfer buffer on first use: the
-    // largest state array of one face (5 doubles per node)
-    staging_bytes = (size_t)(D.E0 + 1) * (D.E1 + 1) * (D.E2 + 1) * 5 * sizeof(double);
-    GCS_TRY(cudaMalloc(&staging, staging_bytes));
-  }
+  if (member_staging() != 0) return -1;
   if (bytes > staging_bytes) {
     set_error("staging too small", "transfer");
     return -1;
@@ -862,17 +858,29 @@ int Context::transfer_array(int f, int kind, int dir, bool upload, double *host)
   return 0;
 }
 
+// A run that shares a grid allocates its transfer buffer on first use: the
+// largest state array of one face (5 doubles per node).
+int Context::member_staging() {
+  if (staging || !owner) return 0;
+  const Dims &D = X.D;
+  const size_t bytes = (size_t)(D.E0 + 1) * (D.E1 + 1) * (D.E2 + 1) * 5 * sizeof(double);
+  GCS_TRY(cudaMalloc(&staging, bytes));
+  staging_bytes = bytes;
+  return 0;
+}
+
 // Moves the state arrays of all faces between the caller's host arrays and
-// the device: per face one gather or scatter kernel and one copy per array,
-// all queued on the context's stream, the faces cycling through as many
-// staging slots as fit, and one wait at the end.  Bound: the host link, and
-// the copies' starts on small grids.  With a wait after every array the
-// drop-in step of 6 x 32x32x48 took 6.3 ms, now 4.5 (95 MB each way); four
-// steps of 6 x 9x9x12 with one download 1.96 ms, now 0.94.
+// the device: the arrays of a face that fit the staging buffer together (all
+// ten in that of a context, the larger ones singly in a member run's) are
+// gathered or scattered by one kernel and copied one by one, everything
+// queued on the context's stream, and one wait at the end.  Bound: the host
+// link, and the copies' starts on small grids.  With a wait after every array
+// the drop-in step of 6 x 32x32x48 took 6.3 ms, now 4.5 (95 MB each way);
+// four steps of 6 x 9x9x12 with one download 1.96 ms, now 0.94.
 int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
   const Dims &D = X.D;
   StateArrays A{};
-  long long total = 0, most = 0;
+  long long total = 0;
   auto add = [&](int a, double *const *p, int comps, int dir) {
     A.comps[a] = comps;
     A.count[a] = 1;
@@ -883,7 +891,6 @@ int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
     for (int q = 0; q < comps; ++q) A.p[a][q] = p[q];
     A.start[a] = total;
     total += A.count[a] * comps;
-    most = std::max(most, A.count[a]);
   };
   add(0, X.S.U, 5, -1);
   add(1, X.S.Uo, 5, -1);
@@ -893,36 +900,35 @@ int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
     add(4 + 2 * d, &X.S.P[d], 1, d);
     add(5 + 2 * d, &X.S.Po[d], 1, d);
   }
-  const size_t bytes = (size_t)total * sizeof(double);
-  if (owner && staging_bytes < bytes) {
-    // runs sharing a grid allocate their transfer buffer on first use
-    if (staging) GCS_TRY(cudaFree(staging));
-    staging = nullptr;
-    staging_bytes = 0;
-    GCS_TRY(cudaMalloc(&staging, bytes));
-    staging_bytes = bytes;
-  }
-  const int slots = (int)std::min<size_t>(kFaces, staging_bytes / bytes);
-  if (slots < 1) {
-    set_error("staging too small", "transfer");
-    return -1;
-  }
-  const dim3 grid(blocks_for(most, 256), 10);
+  if (member_staging() != 0) return -1;
+  const long long room = (long long)(staging_bytes / sizeof(double));
+  auto size = [&](int a) { return A.count[a] * A.comps[a]; };
+  double *stage = (double *)staging;
   for (int f = 0; f < kFaces; ++f) {
-    double *stage = (double *)staging + (long long)(f % slots) * total;
     double *host[10] = {st[f].conserved, st[f].old_conserved, (double *)st[f].cell_magnetic,
                         (double *)st[f].old_cell_magnetic,
                         st[f].face_flux[0], st[f].old_face_flux[0],
                         st[f].face_flux[1], st[f].old_face_flux[1],
                         st[f].face_flux[2], st[f].old_face_flux[2]};
-    if (!upload) k_move_state<false><<<grid, 256, 0, stream>>>(D, f, A, stage);
-    for (int a = 0; a < 10; ++a) {
-      const size_t n = (size_t)A.count[a] * A.comps[a] * sizeof(double);
-      double *s = stage + A.start[a];
-      GCS_TRY(upload ? cudaMemcpyAsync(s, host[a], n, cudaMemcpyHostToDevice, stream)
-                     : cudaMemcpyAsync(host[a], s, n, cudaMemcpyDeviceToHost, stream));
+    for (int first = 0, last; first < 10; first = last) {
+      long long most = 0;
+      for (last = first; last < 10 && A.start[last] + size(last) - A.start[first] <= room;
+           ++last)
+        most = std::max(most, A.count[last]);
+      if (last == first) {
+        set_error("staging too small", "transfer");
+        return -1;
+      }
+      const dim3 grid(blocks_for(most, 256), (unsigned)(last - first));
+      if (!upload) k_move_state<false><<<grid, 256, 0, stream>>>(D, f, A, first, stage);
+      for (int a = first; a < last; ++a) {
+        const size_t n = (size_t)size(a) * sizeof(double);
+        double *s = stage + (A.start[a] - A.start[first]);
+        GCS_TRY(upload ? cudaMemcpyAsync(s, host[a], n, cudaMemcpyHostToDevice, stream)
+                       : cudaMemcpyAsync(host[a], s, n, cudaMemcpyDeviceToHost, stream));
+      }
+      if (upload) k_move_state<true><<<grid, 256, 0, stream>>>(D, f, A, first, stage);
     }
-    if (upload) k_move_state<true><<<grid, 256, 0, stream>>>(D, f, A, stage);
   }
   GCS_TRY(cudaGetLastError());
   GCS_TRY(cudaStreamSynchronize(stream));

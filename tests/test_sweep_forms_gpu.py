@@ -115,3 +115,33 @@ def test_state_round_trip(lib, nr, n, pinned):
     finally:
         lib.gcs_context_destroy(ctx)
 
+
+
+@pytest.mark.parametrize("nr,n", [(9, 9), (26, 11)])
+def test_member_transfer_buffer(lib, nr, n):
+    """A run that shares a grid moves its state through a buffer of five
+    doubles a node of one face, the arrays one by one where they fill it:
+    random states come back bit for bit, and the ensemble grows by no more
+    than those buffers, which its admission estimate leaves out."""
+    driver = (abi.WindDriver * 3)(*[abi.WindDriver(7.0, -420.0, 9e4, -4.0)] * 3)
+    nrs, ns = (C.c_size_t * 3)(nr, nr, nr), (C.c_size_t * 3)(n, n, n)
+    config = abi.EnsembleConfig(3, nrs, ns, driver, 3, 0, 0, 0.5)
+    e = lib.gcs_ensemble_create(C.byref(config))
+    assert e, lib.gcs_last_error()
+    try:
+        before = lib.gcs_ensemble_device_bytes(e)
+        rng = np.random.default_rng(n)
+        for run in range(3):
+            ctx = lib.gcs_ensemble_run_context(e, run)
+            a = HostStorage([nr, n, n], 4, scratch=False)
+            b = HostStorage([nr, n, n], 4, scratch=False)
+            for q in a._keep:
+                q[:] = rng.standard_normal(len(q))
+            assert lib.gcs_context_upload_state(ctx, a.storage) == 0
+            assert lib.gcs_context_download_state(ctx, b.storage, 0) == 0
+            for x, y in zip(a._keep, b._keep):
+                np.testing.assert_array_equal(x, y)
+        grown = lib.gcs_ensemble_device_bytes(e) - before
+        assert 0 < grown <= 2 * 40 * (nr + 9) * (n + 9) * (n + 9)
+    finally:
+        lib.gcs_ensemble_destroy(e)
