@@ -113,6 +113,7 @@ struct Context {
   int transfer_array(int f, int kind, int dir, bool upload, double *host);
   int member_staging();
   int move_state(const gamera_no_storage st[kFaces], bool upload);
+  int queue_state(const gamera_no_storage st[kFaces], bool upload);
   int upload_state(const gamera_no_storage st[kFaces]);
   int download_state(gamera_no_storage st[kFaces], int scratch);
   void reset_status_async();

@@ -878,6 +878,16 @@ int Context::member_staging() {
 // the drop-in step of 6 x 32x32x48 took 6.3 ms, now 4.5 (95 MB each way);
 // four steps of 6 x 9x9x12 with one download 1.96 ms, now 0.94.
 int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
+  cudaGetLastError();  // an earlier call's error, reported by that call
+  const int rc = queue_state(st, upload);
+  // also after an error: the copies queued before it use the caller's arrays
+  const cudaError_t e = cudaStreamSynchronize(stream);
+  if (rc == 0 && e != cudaSuccess) set_error(cudaGetErrorString(e), "transfer");
+  cudaGetLastError();
+  return rc == 0 && e == cudaSuccess ? 0 : -1;
+}
+
+int Context::queue_state(const gamera_no_storage st[kFaces], bool upload) {
   const Dims &D = X.D;
   StateArrays A{};
   long long total = 0;
@@ -931,7 +941,6 @@ int Context::move_state(const gamera_no_storage st[kFaces], bool upload) {
     }
   }
   GCS_TRY(cudaGetLastError());
-  GCS_TRY(cudaStreamSynchronize(stream));
   return 0;
 }
 

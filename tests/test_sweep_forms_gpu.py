@@ -145,3 +145,33 @@ def test_member_transfer_buffer(lib, nr, n):
         assert 0 < grown <= 2 * 40 * (nr + 9) * (n + 9) * (n + 9)
     finally:
         lib.gcs_ensemble_destroy(e)
+
+
+def test_failed_transfer_waits(lib):
+    """A transfer that meets an array it cannot copy (a null pointer, which
+    the copy call refuses) returns -1 only after the copies queued before it:
+    the page-locked arrays they fill are the caller's to free then."""
+    import torch
+    nr, n = 64, 64
+    ctx = lib.gcs_context_create_case(0, nr, n, 1)
+    assert ctx, lib.gcs_last_error()
+    try:
+        want = HostStorage([nr, n, n], 4, pinned=True, scratch=False)
+        got = HostStorage([nr, n, n], 4, pinned=True, scratch=False)
+        assert lib.gcs_context_download_state(ctx, want.storage, 0) == 0
+        for q in got._keep:
+            q.fill_(-1.0)
+        last = C.cast(got.storage[5].old_face_flux[2], C.c_void_p).value
+        got.storage[5].old_face_flux[2] = None
+        rc = lib.gcs_context_download_state(ctx, got.storage, 0)
+        at_return = got._keep[-2].clone()   # face_flux[2], queued just before
+        torch.cuda.synchronize()
+        got.storage[5].old_face_flux[2] = C.cast(last, C.POINTER(C.c_double))
+        assert rc == -1
+        np.testing.assert_array_equal(at_return.numpy(), want._keep[-2].numpy())
+        # the context goes on
+        assert lib.gcs_context_download_state(ctx, got.storage, 0) == 0
+        for x, y in zip(want._keep, got._keep):
+            np.testing.assert_array_equal(x.numpy(), y.numpy())
+    finally:
+        lib.gcs_context_destroy(ctx)
