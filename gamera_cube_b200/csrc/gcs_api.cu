@@ -293,7 +293,7 @@ int run_step(gcs_context *ctx, const gcs::Opts &O, int driver_mode,
     gcs::launch_edge_sync(X, s);
     mk.mark(kSlotEdgeSync);
   }
-  gcs::launch_update(X, O, driver_mode && !post_control, s);
+  gcs::launch_update(X, O, driver_mode && !post_control, s, hk != nullptr && hk->radial);
   mk.mark(kSlotUpdate);
   if (post_control) {
     // the Earth drivers' post-step pressure control with this step's dt,

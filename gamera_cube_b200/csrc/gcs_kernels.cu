@@ -217,6 +217,42 @@ __global__ void k_halo_faces(Dims D, const HaloFace *plan, long long count,
   S.Po[dir][x] = of;
 }
 
+// B recovery of the cells beside the seam faces, after a seam sync of Phi
+// that follows the cell update: one thread per seam face, the two cells
+// beside it on either cube face.  A corner cell has two threads, which store
+// the same values.
+__global__ void k_recover_seams(Dims D, const Seam *seams, DevState S, DevGeom G,
+                                DevStatus *st) {
+  if (failed(st)) return;
+  const long long per = (long long)D.nr * D.n;
+  const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+  if (t >= 12 * per) return;
+  const Seam sm = seams[t / per];
+  const int i = D.g + (int)(t % per) / D.n, along = (int)(t % per) % D.n;
+  const int dalong = sm.reversed ? D.n - 1 - along : along;
+  const long long sdir[3] = {D.stride(0), D.stride(1), 1};
+  for (int side = 0; side < 2; ++side) {
+    const int f = side == 0 ? sm.face : sm.nface;
+    const int axis = side == 0 ? sm.src_axis : sm.dst_axis;
+    const int at = side == 0 ? along : dalong;
+    for (int below = 0; below < 2; ++below) {
+      int x[3] = {i, D.g + at, D.g + at};
+      x[axis] = (side == 0 ? sm.src_b : sm.dst_b) - below;
+      const long long c = f * D.Nn + D.node(x[0], x[1], x[2]);
+      double phi[6], b[3];
+      for (int d = 0; d < 3; ++d) {
+        phi[2 * d] = S.P[d][c];
+        phi[2 * d + 1] = S.P[d][c + sdir[d]];
+      }
+      if (!recover_cell(G, c, phi, b)) {
+        fail(st, kStageRecoverFinal, 0, f, x[0], x[1], x[2]);
+        continue;
+      }
+      for (int m = 0; m < 3; ++m) S.B[m][c] = b[m];
+    }
+  }
+}
+
 // CFL time-step reduction over active cells (nonorthogonal_step.c:449-525)
 // from the stored state; the driver loop's steps reduce it in k_update.
 __global__ void __launch_bounds__(256, 4) k_timestep(Dims D, DevState S, DevGeom G, DevBg BG,
@@ -411,15 +447,22 @@ void launch_edge_sync(const Ctx &X, cudaStream_t s) {
         X.D, X.edge_offsets, X.edge_members, X.n_edge_groups, X.S, X.status);
 }
 
-void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s) {
+void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s,
+                   bool seams_after) {
   const Dims &D = X.D;
   const Tile t = X.tile[kTileCt], tu = X.tile[kTileUpdate];
   for (int d = X.fine_launches ? 0 : -1; d < (X.fine_launches ? 3 : 0); ++d)
     k_ct<<<tile_grid(D.E0 + 1, D.E1 + 1, D.E2 + 1, t), tile_block(t), 0, s>>>(
         D, X.S, O, d < 0 ? 7 : 1 << d, X.params, X.status);
-  if (O.u_mhd) launch_seam_sync(X, 1, s);
+  if (O.u_mhd && !seams_after) launch_seam_sync(X, 1, s);
   k_update<<<tile_grid(D.E0, D.E1, D.E2, tu), tile_block(tu), 0, s>>>(
       D, X.S, X.G, X.BG, O, with_cfl && O.u_mhd, X.params, X.status);
+  if (O.u_mhd && seams_after) {
+    launch_seam_sync(X, 1, s);
+    const long long total = 12LL * D.nr * D.n;
+    k_recover_seams<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(D, X.seams, X.S, X.G,
+                                                                    X.status);
+  }
 }
 
 void launch_timestep(const Ctx &X, const Opts &O, cudaStream_t s) {

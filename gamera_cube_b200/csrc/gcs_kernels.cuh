@@ -90,7 +90,12 @@ void launch_edge_emfs(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_edge_sync(const Ctx &X, cudaStream_t s);
 // CT, the seam sync of Phi, then the cell update with the final recovery;
 // with_cfl: also the CFL reduction of the new state into status.
-void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s);
+// seams_after: the seam sync after the update, then the recovery of the cells
+// beside the seams: where a host callback may have set the two sides of a
+// seam face apart, the momentum update takes each side's own Phi
+// (cubedsphere_step.c:128-152).
+void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s,
+                   bool seams_after = false);
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s);
 // B of every cell as it was before the update that failed (driver mode:
 // launch_next_dt does it on the device).

@@ -396,8 +396,9 @@ __global__ void k_ct(Dims D, DevState S, Opts O, int families, const StepParams 
 // The reference recovers B before the seam sync of Phi for the momentum
 // update and again after it on every cell.  The two sides of a seam face
 // carry the same synced Phi and edge EMFs, so the sync moves Phi by the
-// rounding of the curl only; here it runs before this kernel and one
-// recovery serves both uses, which saves a second pass over the recovery
+// rounding of the curl only; here it runs before this kernel (after it only
+// where a host callback may have set the sides apart) and one recovery serves
+// both uses, which saves a second pass over the recovery
 // map, Phi, U and B0 (264 B per cell).  Bound: HBM (4.9 TB/s).  Four blocks an
 // SM (124 registers): at six, the bound without the recovery, it spills.
 // 6 x 96x96x192, CT, update and recovery: 2.72 -> 1.79 ms a step (six blocks

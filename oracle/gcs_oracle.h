@@ -117,6 +117,8 @@ double gcso_case_default_dt(gcso_case *c);
 double gcso_case_default_ratio(gcso_case *c);
 int gcso_case_local_timestep(gcso_case *c, double *dt);
 int gcso_case_step(gcso_case *c, double ratio, double dt);
+int gcso_case_step_radial(gcso_case *c, double ratio, double dt,
+                          gamera_cs_radial_boundary_function radial, void *context);
 int gcso_case_copy_storage(gcso_case *dst, const gcso_case *src);
 
 #ifdef __cplusplus

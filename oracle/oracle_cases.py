@@ -48,6 +48,8 @@ def lib():
                 ("gcso_case_default_ratio", C.c_double, [C.c_void_p]),
                 ("gcso_case_local_timestep", C.c_int, [C.c_void_p, P(C.c_double)]),
                 ("gcso_case_step", C.c_int, [C.c_void_p, C.c_double, C.c_double]),
+                ("gcso_case_step_radial", C.c_int,
+                 [C.c_void_p, C.c_double, C.c_double, C.c_void_p, C.c_void_p]),
                 ("gcso_case_copy_storage", C.c_int, [C.c_void_p, C.c_void_p]),
                 ("gcso_halo_plan_create", C.c_int, [P(abi.Grid), P(C.c_size_t),
                                                     C.c_size_t, P(C.c_void_p)]),
