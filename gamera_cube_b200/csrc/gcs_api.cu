@@ -161,6 +161,8 @@ enum Slot {
   kSlotEmf, kSlotEdgeSync, kSlotUpdate, kSlotSeamPhiFinal, kSlotRecover,
   kSlotDt, kSlotMi, kSlotCount
 };
+// a second interval of the stage in the same step: time, no call
+constexpr int kSlotGoesOn = 0x100;
 const char *kSlotNames[kSlotCount] = {
     "seam_sync_phi", "halo", "predict", "flux", "seam_sync_flux",
     "edge_emf", "edge_sync", "ct_update", "seam_sync_phi_final",
@@ -293,8 +295,21 @@ int run_step(gcs_context *ctx, const gcs::Opts &O, int driver_mode,
     gcs::launch_edge_sync(X, s);
     mk.mark(kSlotEdgeSync);
   }
-  gcs::launch_update(X, O, driver_mode && !post_control, s, hk != nullptr && hk->radial);
+  gcs::launch_ct(X, O, s);
   mk.mark(kSlotUpdate);
+  const bool seams_after = hk != nullptr && hk->radial != nullptr;
+  if (O.u_mhd && !seams_after) {
+    gcs::launch_seam_sync(X, 1, s);
+    mk.mark(kSlotSeamPhiFinal);
+  }
+  gcs::launch_cells(X, O, driver_mode && !post_control, s);
+  mk.mark(kSlotUpdate | kSlotGoesOn);
+  if (O.u_mhd && seams_after) {
+    gcs::launch_seam_sync(X, 1, s);
+    mk.mark(kSlotSeamPhiFinal);
+    gcs::launch_recover_seams(X, s);
+    mk.mark(kSlotRecover);
+  }
   if (post_control) {
     // the Earth drivers' post-step pressure control with this step's dt,
     // fused with the CFL reduction of the controlled state
@@ -1241,9 +1256,9 @@ int gcs_context_stage_times(gcs_context *ctx, double *ms, long long *calls,
   for (size_t q = 0; q < ctx->event_slot.size(); ++q) {
     float t = 0.0f;
     cudaEventElapsedTime(&t, ctx->events[2 * q], ctx->events[2 * q + 1]);
-    const int slot = ctx->event_slot[q];
+    const int slot = ctx->event_slot[q] & ~kSlotGoesOn;
     ctx->c.stage_ms[slot] += t;
-    ctx->c.stage_calls[slot] += 1;
+    if (!(ctx->event_slot[q] & kSlotGoesOn)) ctx->c.stage_calls[slot] += 1;
   }
   // events are chained (end of one = start of the next): destroy each once
   std::vector<cudaEvent_t> uniq;

@@ -447,22 +447,25 @@ void launch_edge_sync(const Ctx &X, cudaStream_t s) {
         X.D, X.edge_offsets, X.edge_members, X.n_edge_groups, X.S, X.status);
 }
 
-void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s,
-                   bool seams_after) {
+void launch_ct(const Ctx &X, const Opts &O, cudaStream_t s) {
   const Dims &D = X.D;
-  const Tile t = X.tile[kTileCt], tu = X.tile[kTileUpdate];
+  const Tile t = X.tile[kTileCt];
   for (int d = X.fine_launches ? 0 : -1; d < (X.fine_launches ? 3 : 0); ++d)
     k_ct<<<tile_grid(D.E0 + 1, D.E1 + 1, D.E2 + 1, t), tile_block(t), 0, s>>>(
         D, X.S, O, d < 0 ? 7 : 1 << d, X.params, X.status);
-  if (O.u_mhd && !seams_after) launch_seam_sync(X, 1, s);
+}
+
+void launch_cells(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s) {
+  const Dims &D = X.D;
+  const Tile tu = X.tile[kTileUpdate];
   k_update<<<tile_grid(D.E0, D.E1, D.E2, tu), tile_block(tu), 0, s>>>(
       D, X.S, X.G, X.BG, O, with_cfl && O.u_mhd, X.params, X.status);
-  if (O.u_mhd && seams_after) {
-    launch_seam_sync(X, 1, s);
-    const long long total = 12LL * D.nr * D.n;
-    k_recover_seams<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(D, X.seams, X.S, X.G,
-                                                                    X.status);
-  }
+}
+
+void launch_recover_seams(const Ctx &X, cudaStream_t s) {
+  const long long total = 12LL * X.D.nr * X.D.n;
+  k_recover_seams<<<(unsigned)((total + 255) / 256), 256, 0, s>>>(X.D, X.seams, X.S, X.G,
+                                                                  X.status);
 }
 
 void launch_timestep(const Ctx &X, const Opts &O, cudaStream_t s) {
@@ -501,7 +504,9 @@ void launch_step(const Ctx &X, const Opts &O, int driver_mode,
     launch_emf(X, O, s);
     launch_edge_sync(X, s);
   }
-  launch_update(X, O, driver_mode, s);
+  launch_ct(X, O, s);
+  if (O.u_mhd) launch_seam_sync(X, 1, s);
+  launch_cells(X, O, driver_mode, s);
   if (driver_mode) launch_next_dt(X, O.dt_fraction, s);
 }
 

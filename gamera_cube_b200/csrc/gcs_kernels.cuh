@@ -88,14 +88,14 @@ void launch_emf(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_face_velocities(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_edge_emfs(const Ctx &X, const Opts &O, cudaStream_t s);
 void launch_edge_sync(const Ctx &X, cudaStream_t s);
-// CT, the seam sync of Phi, then the cell update with the final recovery;
-// with_cfl: also the CFL reduction of the new state into status.
-// seams_after: the seam sync after the update, then the recovery of the cells
-// beside the seams: where a host callback may have set the two sides of a
-// seam face apart, the momentum update takes each side's own Phi
-// (cubedsphere_step.c:128-152).
-void launch_update(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s,
-                   bool seams_after = false);
+// The last stages: CT; the seam sync of Phi (launch_seam_sync); the cell
+// update with the final recovery, with_cfl also with the CFL reduction of the
+// new state into status.  Where a host callback may have set the two sides of
+// a seam face apart the sync comes after the update, which takes each side's
+// own Phi (cubedsphere_step.c:128-152), and launch_recover_seams after that.
+void launch_ct(const Ctx &X, const Opts &O, cudaStream_t s);
+void launch_cells(const Ctx &X, const Opts &O, int with_cfl, cudaStream_t s);
+void launch_recover_seams(const Ctx &X, cudaStream_t s);
 void launch_next_dt(const Ctx &X, double fraction, cudaStream_t s);
 // B of every cell as it was before the update that failed (driver mode:
 // launch_next_dt does it on the device).

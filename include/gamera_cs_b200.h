@@ -330,7 +330,10 @@ int gcs_context_set_profiling(gcs_context *ctx, int on);
  * faster of the two on B200); the two give the same fluxes bit for bit. */
 int gcs_context_set_flux_staging(gcs_context *ctx, int on);
 /* Accumulated device milliseconds and launch counts per stage since
- * profiling was switched on; returns the number of stages written. */
+ * profiling was switched on; returns the number of stages written.
+ * "ct_update" is the CT curl and the cell update; the update recovers B and
+ * reduces the CFL step in the same kernel, so "recover_cfl" has only the
+ * recovery beside the seams after a host radial callback. */
 int gcs_context_stage_times(gcs_context *ctx, double *ms, long long *calls,
                             int capacity);
 const char *gcs_stage_name(int stage_slot);

@@ -175,3 +175,24 @@ def test_failed_transfer_waits(lib):
             np.testing.assert_array_equal(x.numpy(), y.numpy())
     finally:
         lib.gcs_context_destroy(ctx)
+
+
+def test_stage_times_name_what_ran(lib):
+    """Profiled steps: every stage of the step has one call a step and its own
+    time; recover_cfl, whose work is the update kernel's, has none."""
+    ctx = lib.gcs_context_create_case(2, 12, 9, 1)
+    assert ctx, lib.gcs_last_error()
+    try:
+        o, t = abi.AdvanceOptions(), abi.TimestepOptions()
+        lib.gcs_case_options(2, C.byref(o), C.byref(t))
+        assert lib.gcs_context_set_profiling(ctx, 1) == 0
+        assert lib.gcs_context_run(ctx, C.byref(o), C.byref(t), 0.5, 3, 0) == 0
+        ms, calls = (C.c_double * 16)(), (C.c_longlong * 16)()
+        count = lib.gcs_context_stage_times(ctx, ms, calls, 16)
+        got = {lib.gcs_stage_name(q).decode(): (calls[q], ms[q]) for q in range(count)}
+        idle = {"recover_cfl", "mi_coupling"}
+        for name, (n, time) in got.items():
+            assert n == (0 if name in idle else 3), got
+            assert (time > 0.0) == (name not in idle), got
+    finally:
+        lib.gcs_context_destroy(ctx)
