@@ -114,7 +114,7 @@ bool make_opts(const gamera_no_advance_options *o, bool have_background,
   O.e_rho_floor = e.density_floor;
   O.e_pdm = e.pdm_coefficient;
   O.e_diff = e.diffusion_coefficient;
-  O.e_c = e.light_speed;
+  O.e_ic2 = e.use_boris ? 1.0 / (e.light_speed * e.light_speed) : 0.0;
   O.e_cfl = e.cfl;
   O.e_boris = e.use_boris;
   O.e_bg = e.use_background;

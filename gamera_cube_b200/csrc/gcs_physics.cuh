@@ -545,18 +545,19 @@ __device__ inline int emergency_diffusion(FluidFlux<T> *fl, const PrimT<T> st[2]
 
 // nonorthogonal_operators.c:144-182 (length > DBL_MIN checked at set-up).
 // Speeds from squares: |v_t| and, with the Boris correction, c va / hypot(c,
-// va) = c |b_t| / sqrt(c^2 rho + |b_t|^2), else |b_t| / sqrt(rho): two square
+// va) = |b_t| / sqrt(rho + |b_t|^2 / c^2), else |b_t| / sqrt(rho): two square
 // roots and a division where the reference takes three hypotenuses, a root
-// and two divisions.  limit = cfl / dt.
+// and two divisions.  ic2 = 1 / c^2 with the Boris correction (rounded to 0
+// where c^2 overflows, which leaves the limit of large c), else 0; limit =
+// cfl / dt.
 template <typename T>
 __device__ __forceinline__ int edge_emf(T vt1, T vt2, T bt1, T bt2, T jump, T rho, T length,
-                                        T diffusion, bool use_boris, T c, T limit, T *emf) {
+                                        T diffusion, T ic2, T limit, T *emf) {
   const bool ok = isfinite(vt1) && isfinite(vt2) && isfinite(bt1) && isfinite(bt2) &&
                   isfinite(jump) && isfinite(rho) && rho > Num<T>::tiny;
   const T flow = Num<T>::sqrt0(vt1 * vt1 + vt2 * vt2);
   const T b2 = bt1 * bt1 + bt2 * bt2;
-  const T va = use_boris ? c * Num<T>::sqrt0(b2 * Num<T>::rcp(c * c * rho + b2))
-                         : Num<T>::sqrt0(b2 * Num<T>::rcp(rho));
+  const T va = Num<T>::sqrt0(b2 * Num<T>::rcp(rho + b2 * ic2));
   const T speed = fmin(flow + va, limit * length);
   const T ideal = -(vt1 * bt2 - vt2 * bt1);
   *emf = (ideal + diffusion * speed * jump) * length;

@@ -196,3 +196,39 @@ def test_stage_times_name_what_ran(lib):
             assert (time > 0.0) == (name not in idle), got
     finally:
         lib.gcs_context_destroy(ctx)
+
+
+def test_large_light_speeds(lib):
+    """The Boris correction at light speeds whose square overflows in FP32 or
+    FP64 (it does nothing there): one step against the restatement to 1e-12,
+    and one FP32-bulk step against the FP64 one to 1e-5 of the largest EMF, a
+    few dozen FP32 roundings (an Alfven speed lost to the overflow is 4e-5
+    off in FP32, 1e-4 in FP64)."""
+    ref, gpu = oracle_cases.pair("wind", 12, 9, 5)
+    dt = 0.4 * ref.local_timestep()
+    ctx = lib.gcs_context_create(gpu.grid, gpu.active, gpu.ghost)
+    assert ctx, lib.gcs_last_error()
+    try:
+        assert lib.gcs_context_upload_background(ctx, gpu.background) == 0
+        for light_speed in (10.0, 1e20, 1e160):
+            for case in (ref, gpu):
+                o = case.options[0]
+                for group in (o.stress, o.emf, o.update):
+                    assert group.use_boris
+                    group.light_speed = light_speed
+            done = [HostStorage(list(gpu.active), gpu.ghost) for _ in range(2)]
+            for bulk in (0, 1):
+                assert lib.gcs_context_set_precision(ctx, bulk) == 0
+                assert lib.gcs_context_upload_state(ctx, gpu.storage) == 0
+                assert lib.gcs_context_step(ctx, gpu.options, 0.0, dt) == 0
+                assert lib.gcs_context_download_state(ctx, done[bulk].storage, 1) == 0
+            ref.copy_from(gpu)
+            assert ref.step(0.0, dt) == 0
+            bad = {k: v for k, v in compare_state(done[0], ref).items() if not v[0] <= 1e-12}
+            assert not bad, (light_speed, bad)
+            for f in range(6):
+                for e in range(3):
+                    x, y = (s.arrays(f)["edge_emf%d" % e] for s in done)
+                    assert np.abs(x - y).max() <= 1e-5 * np.abs(x).max(), light_speed
+    finally:
+        lib.gcs_context_destroy(ctx)
