@@ -7,6 +7,18 @@
 namespace gcs {
 
 void launch_flux_f32(const Ctx &X, const Opts &O, int i0, int i1, cudaStream_t s) {
+  if (i1 <= X.D.g || i0 > X.D.g + X.D.nr) return;
+  // options outside FP32 fail the step here: the sweep reads 1 / (gamma - 1)
+  // and 1 / c^2, not gamma and c
+  const float gamma = (float)O.s_gamma, c = (float)O.s_c;
+  if (!(gamma > 1.0f) || !isfinite(gamma)) {
+    launch_set_failure(X, kStageKineticFluid, 0, s);
+    return;
+  }
+  if (O.s_mhd && O.s_boris && !(c > FLT_MIN && isfinite(c))) {
+    launch_set_failure(X, kStageKineticMaxwell, 0, s);
+    return;
+  }
   Sweeps<float>::flux(X, X.B32, O, i0, i1, s);
 }
 void launch_face_velocity_f32(const Ctx &X, const Opts &O, int i0, int i1,

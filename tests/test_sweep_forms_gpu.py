@@ -220,15 +220,44 @@ def test_large_light_speeds(lib):
             for bulk in (0, 1):
                 assert lib.gcs_context_set_precision(ctx, bulk) == 0
                 assert lib.gcs_context_upload_state(ctx, gpu.storage) == 0
+                if bulk and light_speed > 3e38:
+                    break   # not an FP32 number: test_options_outside_fp32
                 assert lib.gcs_context_step(ctx, gpu.options, 0.0, dt) == 0
                 assert lib.gcs_context_download_state(ctx, done[bulk].storage, 1) == 0
             ref.copy_from(gpu)
             assert ref.step(0.0, dt) == 0
             bad = {k: v for k, v in compare_state(done[0], ref).items() if not v[0] <= 1e-12}
             assert not bad, (light_speed, bad)
+            if light_speed > 3e38:
+                continue
             for f in range(6):
                 for e in range(3):
                     x, y = (s.arrays(f)["edge_emf%d" % e] for s in done)
                     assert np.abs(x - y).max() <= 1e-5 * np.abs(x).max(), light_speed
+    finally:
+        lib.gcs_context_destroy(ctx)
+
+
+@pytest.mark.parametrize("gamma,light_speed,stage", [
+    (5.0 / 3.0, 10.0, 0),
+    (1.0 + 1e-9, 10.0, 4),     # 1 in FP32
+    (5.0 / 3.0, 1e39, 5),      # infinite in FP32
+    (5.0 / 3.0, 1e-39, 5),     # below the smallest normal FP32 number
+])
+def test_options_outside_fp32(lib, gamma, light_speed, stage):
+    """gamma and c that FP32 cannot hold fail a step with FP32 layers, with the
+    flux sweep's stage codes."""
+    ctx = lib.gcs_context_create_case(2, 12, 9, 1)
+    assert ctx, lib.gcs_last_error()
+    try:
+        o, t = abi.AdvanceOptions(), abi.TimestepOptions()
+        lib.gcs_case_options(2, C.byref(o), C.byref(t))
+        o.stress.gamma = o.update.gamma = gamma
+        for group in (o.stress, o.emf, o.update):
+            group.light_speed = light_speed
+        assert lib.gcs_context_set_precision(ctx, 1) == 0
+        rc = lib.gcs_context_step(ctx, C.byref(o), 0.0, 1e-6)
+        assert lib.gcs_context_failure(ctx, None, None, None, None, None) == stage
+        assert rc == (0 if stage == 0 else -1)
     finally:
         lib.gcs_context_destroy(ctx)
