@@ -261,11 +261,16 @@ __device__ __forceinline__ void copy16(unsigned dst, const void *src) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src));
 }
 
-// Inboxes carry kInboxPad slots before the first longitude and as many and a
-// group after the last, so a sending lane stores its off-grid steps too
-// (columns -7 .. np + 37 less the lane), without a test.
-constexpr int kInboxPad = 32;
-__host__ __device__ constexpr int inbox_len(int np) { return np + 2 * kInboxPad + kGroup; }
+// Inboxes carry kInboxPad slots before the first longitude and as many after
+// the last, so lanes send, take and read off-grid steps without a test.  A
+// sweep's columns are 0 .. np + 37 (forward) or np + 30 .. -7 (reverse), the
+// last group filled up with steps past the np + 31.  By longitude, lane 31
+// sends to its column less 31 (forward), lane 0 to its column (reverse); the
+// receiver takes its column (forward, up to np + 37) or its column less 31
+// (reverse, down to -38).  The pole edges are read by column.
+constexpr int kInboxPad = 40;
+static_assert(kInboxPad >= 31 + kGroup - 1, "the last group's steps stay inside an inbox");
+__host__ __device__ constexpr int inbox_len(int np) { return np + 2 * kInboxPad; }
 
 // Shared memory of the sweep warps of one CTA: per warp a prefetch ring and
 // the two inboxes (the row below the block for the forward sweep, above it
