@@ -19,10 +19,15 @@ template <typename T> struct Num;
 template <> struct Num<double> {
   static constexpr double tiny = DBL_MIN;
 #ifdef __CUDACC__
-  // 1 / x and 1 / sqrt(x) of a finite normal x: the hardware's 20-bit
-  // approximation and one third-order (Householder) step, within 1 ulp; no
-  // special cases and no slow path, where a division or square root brings
-  // both into every face's instruction stream.
+  // 1 / x and 1 / sqrt(x): the hardware's approximation (20 bits or more) and
+  // one step of Householder's method of third order, the series of the exact
+  // correction in the residual e cut after e^2:
+  //   1 / x = r / (1 - e) ~ r (1 + e + e^2),                  e = 1 - x r
+  //   1 / sqrt(x) = y (1 - e)^-1/2 ~ y (1 + e/2 + 3 e^2 / 8),  e = 1 - x y^2
+  // Within 1 ulp for 2^-1022 <= |x| <= 2^1021 (rcp) and normal x > 0
+  // (rsqrt_), tests/test_sweep_math_gpu.py; 0, infinities and results below
+  // the normal numbers are not handled, which keeps the special cases and the
+  // slow path of a division or root out of every face's instruction stream.
   __device__ static double rcp(double x) {
     double r;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(r) : "d"(x));
@@ -80,8 +85,8 @@ template <> struct Num<float> {
 // polynomial in t = (|x| - 4) / (|x| + 4), the transformation of Shepherd and
 // Laframboise (Math. Comp. 36, 1981); both polynomials interpolate the
 // functions (50 digits) at Chebyshev points, erfcx over |x| <= 28, beyond
-// which exp(-x^2) is 0.  Largest error over |x| <= 26: 2.4 units of 2^-52
-// relative (erfc), 0.8 (exp).
+// which exp(-x^2) is 0.  Finite x; largest error over |x| <= 26: 2.4 units of
+// 2^-52 relative (erfc), 0.8 (exp).
 __device__ inline void Num<double>::erfc_exp(double x, double *erfc_x, double *exp_mx2) {
   constexpr double kQ[23] = {
       1.0959956610004911183, -0.97654872908088212578, 0.77320870226523745861,
