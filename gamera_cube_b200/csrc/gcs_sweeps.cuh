@@ -531,6 +531,15 @@ inline dim3 boxes_grid(const Boxes &X, int groups, Tile t) {
   for (int q = 0; q < 3; ++q) points = max(points, X.b[q].nj * X.b[q].nk);
   return dim3((unsigned)((points + t.bx - 1) / t.bx), 3u * (unsigned)groups, kFaces);
 }
+// A sweep's tile: grid.y holds the layer groups of three families in at most
+// 65535 blocks, so a grid of more layers than that gets taller tiles.
+inline Tile sweep_tile(Tile t, int layers) {
+  while (3LL * ((layers + t.by - 1) / t.by) > 65535 && t.bx % 2 == 0) {
+    t.bx /= 2;
+    t.by *= 2;
+  }
+  return t;
+}
 template <typename T>
 struct Sweeps {
   static void flux(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
@@ -546,7 +555,7 @@ struct Sweeps {
         launch_flux_tma<2, T>(X, B, O, a, a + n, s);
       return;
     }
-    const Tile t = X.tile[kTileFlux];
+    const Tile t = sweep_tile(X.tile[kTileFlux], D.E0 + 1);
     Boxes b;
     for (int d = 0; d < 3; ++d)
       b.b[d] = Box{0, D.g, D.g, D.n + (d == 1), D.n + (d == 2), 0};
@@ -562,7 +571,7 @@ struct Sweeps {
                   cudaStream_t s) {
     const Dims &D = X.D;
     // face velocities: family a, edge family e=(a+2)%3 active, a faces, bb all
-    const Tile t = X.tile[kTileFaceVelocity];
+    const Tile t = sweep_tile(X.tile[kTileFaceVelocity], D.E0 + 1);
     Boxes b;
     int lo[3], hi[3];
     for (int a = 0; a < 3; ++a) {
@@ -592,7 +601,7 @@ struct Sweeps {
   static void edge(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
                    cudaStream_t s) {
     const Dims &D = X.D;
-    const Tile t = X.tile[kTileEdgeEmf];
+    const Tile t = sweep_tile(X.tile[kTileEdgeEmf], D.E0 + 1);
     Boxes b;
     int lo[3], hi[3];
     for (int e = 0; e < 3; ++e) {

@@ -261,3 +261,26 @@ def test_options_outside_fp32(lib, gamma, light_speed, stage):
         assert rc == (0 if stage == 0 else -1)
     finally:
         lib.gcs_context_destroy(ctx)
+
+
+def test_more_layers_than_a_grid_dimension(lib):
+    """22,000 radial layers: three families of them are more than grid.y's
+    65535 blocks of one layer.  The step runs, and the uniform state keeps its
+    CFL step."""
+    import torch
+    if torch.cuda.mem_get_info()[0] < 90e9:
+        pytest.skip("needs 75 GB of device memory")
+    ctx = lib.gcs_context_create_case(0, 22000, 9, 1)
+    assert ctx, lib.gcs_last_error()
+    try:
+        o, t = abi.AdvanceOptions(), abi.TimestepOptions()
+        lib.gcs_case_options(0, C.byref(o), C.byref(t))
+        before, after = C.c_double(), C.c_double()
+        assert lib.gcs_context_timestep(ctx, C.byref(t), C.byref(before)) == 0
+        assert lib.gcs_context_step(ctx, C.byref(o), 0.0, 0.4 * before.value) == 0
+        assert lib.gcs_context_timestep(ctx, C.byref(t), C.byref(after)) == 0
+        # fluxes of 1 over layers 2e-5 thick cancel to rounding: 1e5 x 1e-16 x
+        # a few dozen operations a step
+        assert abs(after.value / before.value - 1.0) <= 1e-9
+    finally:
+        lib.gcs_context_destroy(ctx)
