@@ -374,11 +374,15 @@ int flux_tma_blocks() {
   return blocks;
 }
 
+// The form without tangents (kOrtho) exists in FP64 only.
+template <bool kOrtho, typename T>
+bool flux_tma_ready() {
+  return flux_tma_blocks<0, kOrtho, T>() > 0 && flux_tma_blocks<1, kOrtho, T>() > 0 &&
+         flux_tma_blocks<2, kOrtho, T>() > 0;
+}
 template <typename T>
 int prepare_flux_tma() {
-  return (flux_tma_blocks<0, true, T>() > 0 && flux_tma_blocks<1, true, T>() > 0 &&
-          flux_tma_blocks<2, true, T>() > 0 && flux_tma_blocks<0, false, T>() > 0 &&
-          flux_tma_blocks<1, false, T>() > 0 && flux_tma_blocks<2, false, T>() > 0) ? 0 : -1;
+  return flux_tma_ready<false, T>() && flux_tma_ready<sizeof(T) == 8, T>() ? 0 : -1;
 }
 
 // Launch of the staged flux sweep of direction d over [i0, i1).
@@ -399,14 +403,15 @@ void launch_flux_tma(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int 
       launch_set_failure(X, kStageTileCopy, d, s);
       return;
     }
-  const bool ortho = X.ortho && sizeof(T) == 8;  // as the per-face sweep
-  const int blocks = ortho ? flux_tma_blocks<d, true, T>() : flux_tma_blocks<d, false, T>();
+  constexpr bool kFp64 = sizeof(T) == 8;  // FP32 reads the tangents, as per face
+  const bool ortho = X.ortho && kFp64;
+  const int blocks = ortho ? flux_tma_blocks<d, kFp64, T>() : flux_tma_blocks<d, false, T>();
   if (blocks <= 0) {
     launch_set_failure(X, kStageTileCopy, d, s);
     return;
   }
   const long long grid = L.count < blocks ? L.count : blocks;
-  (ortho ? k_flux_tma<d, true, T> : k_flux_tma<d, false, T>)
+  (ortho ? k_flux_tma<d, kFp64, T> : k_flux_tma<d, false, T>)
       <<<(unsigned)grid, Sh::THREADS, Sh::SMEM, s>>>(maps, D, X.S, B, O, X.status, L);
 }
 

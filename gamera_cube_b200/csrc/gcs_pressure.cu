@@ -45,40 +45,6 @@ __device__ inline unsigned long long warp_max(unsigned long long v) {
   return v;
 }
 
-// CFL candidate of one active cell (nonorthogonal_step.c:449-525, the same
-// arithmetic as the update kernel's fused CFL reduction): false when the
-// reference fails the cell.
-__device__ inline bool cfl_candidate(const double u[5], const double bn[3], const double *b0,
-                                     double cflmin, const Opts &O, double *cand) {
-  Prim p;
-  if (cons_to_prim(u, O.t_gamma, O.t_rho_floor, O.t_p_floor, &p)) return false;
-  const double cs = sqrt(O.t_gamma * p.p / p.rho);
-  double va = 0.0;
-  if (O.t_mhd) {
-    double bx = bn[0], by = bn[1], bz = bn[2];
-    if (b0) {
-      bx = bn[0] + b0[0];
-      by = bn[1] + b0[1];
-      bz = bn[2] + b0[2];
-    }
-    double s2 = 0.0;
-    s2 += bx * bx;
-    s2 += by * by;
-    s2 += bz * bz;
-    va = sqrt(s2) / sqrt(p.rho);
-    if (O.t_boris) va = O.t_c * va / hypot(O.t_c, va);
-  }
-  double v2 = 0.0;
-  v2 += p.vx * p.vx;
-  v2 += p.vy * p.vy;
-  v2 += p.vz * p.vz;
-  const double speed = sqrt(v2) + hypot(cs, va);
-  const double c0 = O.t_cfl * cflmin / speed;
-  if (!isfinite(c0) || c0 <= 0.0) return false;
-  *cand = c0;
-  return true;
-}
-
 // nonorthogonal_step.c:95-152, one thread per active cell; dt from the step
 // parameters when prm is set (the device driver loop), else `dt`.  In the
 // driver loop (with_cfl) the kernel also reduces the CFL step of the
@@ -147,10 +113,10 @@ __global__ void __launch_bounds__(256) k_pressure_control(
     if (with_cfl) {
       // the cell as stored now: controlled, or unchanged
       const double bn[3] = {S.B[0][c], S.B[1][c], S.B[2][c]};
-      double b0[3];
+      double b0[3] = {0.0, 0.0, 0.0};
       if (O.t_bg)
         for (int m = 0; m < 3; ++m) b0[m] = BG.b0[m][c];
-      if (!cfl_candidate(u, bn, O.t_bg ? b0 : nullptr, G.cflmin[c], O, &cand)) {
+      if (!cfl_step(O, u, bn, b0, G.cflmin[c], &cand)) {
         cand = DBL_MAX;
         fail(status, kStageTimestep, 0, f, D.g + i, D.g + j, D.g + k);
       }

@@ -2,8 +2,11 @@
 // type T of the sweeps.
 //
 // T = double is the plain FP64 path: every array of the Bulk<double> view
-// is the FP64 array of DevState/DevGeom/DevBg and the arithmetic is the
-// reference's (gcs_kernels.cu, built without FMA contraction).
+// is the FP64 array of DevState/DevGeom/DevBg.  The flux, face-velocity and
+// edge-EMF sweeps (gcs_kernels_fp64.cu) are built with FMA contraction and
+// take reciprocals, roots and the erfc/exp pair of gcs_physics.cuh: the
+// reference's formulas to a few roundings.  The predictor, CT and cell update
+// (gcs_kernels.cu) keep the reference's operations, without contraction.
 // T = float is the FP32-bulk path (gcs_kernels_bulk.cu, built with FMA):
 // the predictor still advances the FP64 state and also writes FP32 copies
 // of the cell primitives, cell B, face normal fields and EMF weights; the
@@ -139,7 +142,7 @@ struct SweepOccupancy<float> {
 // Bound: FP64 issue and latency at 16 warps an SM (128 registers; 3 to 5
 // blocks of 128 measured within 2 %).  All directions in one launch find a
 // layer's cells in L2 (a launch each: 3.81 against 3.67 ms).  6 x 96x96x192:
-// 4.46 -> 3.02 ms a step, 2774 -> 1700 instructions a face.
+// 4.46 -> 3.01 ms a step, 2774 -> 1740 instructions a face.
 template <bool kOrtho, typename T>
 __global__ void __launch_bounds__(128, SweepOccupancy<T>::flux)
     k_flux(Dims D, DevState S, const __grid_constant__ Bulk<T> B, Opts O, DevStatus *st,
@@ -561,10 +564,11 @@ struct Sweeps {
       b.b[d] = Box{0, D.g, D.g, D.n + (d == 1), D.n + (d == 2), 0};
     const int lo[3] = {D.g, D.g, D.g}, hi[3] = {D.g + D.nr + 1, D.g + D.nr, D.g + D.nr};
     // FP32 reads the tangents: its rounded frame is not orthonormal to FP32
-    const bool ortho = X.ortho && sizeof(T) == 8;
+    constexpr bool kFp64 = sizeof(T) == 8;
+    const bool ortho = X.ortho && kFp64;
     const int groups = clamp_boxes(b, lo, hi, i0, i1, t);
     if (groups > 0)
-      (ortho ? k_flux<true, T> : k_flux<false, T>)
+      (ortho ? k_flux<kFp64, T> : k_flux<false, T>)
           <<<boxes_grid(b, groups, t), tile_block(t), 0, s>>>(D, X.S, B, O, X.status, b);
   }
   static void emf(const Ctx &X, const Bulk<T> &B, const Opts &O, int i0, int i1,
