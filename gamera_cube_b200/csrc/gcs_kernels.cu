@@ -5,11 +5,16 @@
 // six-face step (cubedsphere/cubedsphere_step.c:48-152):
 //   seam Phi sync -> cell halo (+radial outflow) -> face halo -> predictor
 //   -> face-flux sweeps -> seam flux sync -> face velocities -> edge EMF
-//   -> edge EMF group sync -> CT -> cell update (Reynolds + Boris/Maxwell)
-//   -> seam Phi sync -> B recovery (+ CFL reduction in driver mode).
-// Each kernel returns early once an earlier stage has recorded a failure,
-// so stages after a failing one leave the state untouched, as in the
-// reference which returns -1 from the first failing stage.
+//   -> edge EMF group sync -> CT -> seam Phi sync -> cell update (Reynolds +
+//   Boris/Maxwell) with the final B recovery (+ CFL reduction in driver mode).
+// The reference syncs Phi after the update and recovers B once more; so does
+// this step where a host callback may have set the two sides of a seam face
+// apart (k_update, gcs_sweeps.cuh).
+// Kernels return without storing once an earlier stage has recorded a
+// failure, so stages after a failing one leave the state untouched, as in the
+// reference which returns -1 from the first failing stage; a failed update
+// also takes back the B that its kernel has stored (undo_magnetic).  Phi on
+// the seam faces has been synced by then.
 #include "gcs_kernels.cuh"
 #include "gcs_kernel_util.cuh"
 #include "gcs_physics.cuh"

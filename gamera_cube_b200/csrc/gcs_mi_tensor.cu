@@ -31,7 +31,7 @@
 // multiply-adds).  Two rows per lane make np + R / 2 steps of the chain where
 // one row per lane would make np + R with a chain one multiply-add shorter.
 // Measured at 361 x 181 (449 iterations): one warp sweeping whole
-// anti-diagonals 167-175 ms, this 93 ms.  A group of eight steps takes some 1,010
+// anti-diagonals 167-175 ms, this 91-100 ms.  A group of eight steps takes some 1,010
 // to 1,230 cycles: 730 for the steps, 230 for issuing the copies ahead, 150
 // for taking the neighbouring block's row.  Slower: the copies and operand
 // loads spread between the steps (105 ms), groups of four (115), a second
@@ -115,11 +115,11 @@ struct TSys {
   double2 *cb;  // (up, lu) / dg: reverse sweep
   double *pe;   // pole edge coefficients (np)
   double *pole_sum;
-  int *fault;   // set when a sweep copy never arrived
+  int *fault;   // set when a neighbouring block's or band's value never arrived
   gamera_mi_solver_stats *stats;
-  int *status;  // 0 converged, 1 not converged, 2 non-finite FAC, 3 sweep copy lost
+  int *status;  // 0 converged, 1 not converged, 2 non-finite FAC, 3 sweep value lost
   int colored;  // 1: multicolour SSOR by the whole cluster instead of the wavefront
-  int band;     // rows per band of the band-pipelined sweeps (0: one sweep warp)
+  int band;     // rows per band of the band-pipelined sweeps (0: blocks of 64 rows)
   int nbands;   // bands (CTAs 0 .. nbands - 1 sweep)
 };
 
@@ -199,9 +199,9 @@ __device__ __forceinline__ unsigned smem_u32(const void *p) {
 // memory (a distributed-shared-memory store) and the receiving lane polls
 // its own copy until the value replaces the empty mark.  The bands thus
 // form a pipeline in which each CTA trails the previous one by about hb
-// steps, and every point is updated from exactly the operands of the
-// single-warp wavefront, in the same order: the two schedules give
-// identical results.
+// steps, and every point is updated from exactly the operands of the row
+// blocks' wavefront, in the same order: the two schedules give identical
+// results.
 //
 // Shared memory of a band (per CTA): the forward and reverse coefficient
 // pairs and the sweep values at band diagonal d = j + l, slot d h + l (a
@@ -1331,12 +1331,13 @@ gcs_mi_tensor_plan *plan_create(const gamera_mi_solver_config *c) {
     return nullptr;
   }
   // band schedule: one band of at most 32 rows per CTA, its coefficient
-  // tables in shared memory beside the ring's room.  The default on grids
-  // of fewer than 17 longitudes, where the one-warp sweep cannot move its
-  // diagonals in groups of 8 and the band pipeline measured faster (B200:
-  // 70 x 12 7.5 -> 5.7 ms, 12 x 8 1.3 -> 0.4 ms, 40 x 5 7.6 -> 2.1 ms); on
-  // wider grids the one warp is faster (181 x 361: 163 against 224 ms) and
-  // the band schedule is available through gcs_mi_tensor_plan_set_schedule.
+  // tables in shared memory beside the ring's room.  It is what plans of
+  // fewer than 17 longitudes report and start with, from the time when the
+  // sweeps of whole anti-diagonals were slower there.  The row blocks are the
+  // faster on every grid measured (solves on B200, blocks against bands:
+  // 12 x 8 0.36 and 0.38 ms, 40 x 5 1.23 and 2.17, 70 x 12 3.2 and 5.3,
+  // 300 x 16 34 and 95, 60 x 17 2.0 and 5.0, 181 x 361 91 and 212);
+  // gcs_mi_tensor_plan_set_schedule picks.
   if (p->csize >= 2) {
     const int h = (R + p->csize - 1) / p->csize;
     const size_t need = std::max(p->smem, band_smem(h, np));
@@ -1485,7 +1486,7 @@ int gamera_mi_solve_conductance_tensor(const gamera_mi_solver_config *config,
     return -1;
   }
   if (status == 3) {
-    set_api_error("MI tensor solve: a sweep copy did not arrive within the wait limit");
+    set_api_error("MI tensor solve: a neighbouring row's value did not arrive within the wait limit");
     return -1;
   }
   if (stats) *stats = s;

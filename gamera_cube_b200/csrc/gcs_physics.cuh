@@ -1,11 +1,15 @@
 // Device-side MHD point operators of the cubed-sphere step.
 //
-// Every function restates one reference operator with the same operation
-// order (so the FP64 path tracks the CPU reference to round-off); the cited
-// lines are in the GAMERA-Cube project.  The exceptions are marked where they
-// occur: a repeated divisor applied as one reciprocal, sqrt(pi lambda) taken
-// as sqrt(pi) sqrt(lambda), each a change in the last bit.  Functions return
-// 0 on success and a nonzero value where the reference returns -1.
+// Every function restates one reference operator; the cited lines are in the
+// GAMERA-Cube project.  The state conversions, the Boris and Maxwell updates
+// and the FP32 reconstruction keep the reference's operation order.  The
+// FP64 sweep operators (reconstruction, limiter, kinetic fluxes, HOGS,
+// emergency diffusion, edge EMF) rearrange theirs -- reciprocals for repeated
+// divisors, shared weights, speeds compared or formed from squares, one
+// exponential for erfc and exp -- as noted at each, and track the reference
+// to a few roundings; of these the FP32 ones share the limiter, the edge
+// speeds, the emergency test and 1 / c^2.  Functions return 0 on success and
+// a nonzero value where the reference returns -1.
 #pragma once
 
 #include <cfloat>

@@ -148,8 +148,9 @@ int gamera_mi_solve_constant_pedersen(const gamera_mi_solver_config *config,
 int gamera_mi_apply_conductance_tensor(const gamera_mi_solver_config *config,
                                        const double *pedersen, const double *hall,
                                        const double *potential_v, double *result);
-/* nonorthogonal_mi.h:99-102.  SSOR-BiCGStab on one thread-block
- * cluster: the SSOR sweeps run as wavefronts, a warp to 64 rows; at most 512 interior colatitude rows. */
+/* nonorthogonal_mi.h:99-102.  SSOR-BiCGStab on one thread-block cluster:
+ * the SSOR sweeps run as wavefronts, a warp to 64 rows; at most 512 interior
+ * colatitude rows. */
 int gamera_mi_solve_conductance_tensor(const gamera_mi_solver_config *config,
                                        const double *fac_a_m2, const double *pedersen,
                                        const double *hall, double *potential_v,
@@ -579,8 +580,10 @@ int gcs_context_tile(const gcs_context *ctx, int family, int *bx, int *by);
  * recovery/CFL families, times every candidate tile (`repetitions`
  * launches each, CUDA events on the context stream) on the context's
  * current state and keeps the fastest.  These kernels write only per-step
- * scratch, so the state is unchanged; CT and the cell update keep their
- * tile.  best_ms / default_ms (nullable, GCS_TILE_FAMILIES entries, 0 for
+ * scratch, so the state is unchanged; CT and the cell update, which also
+ * recovers B and reduces the CFL step in a driver step, keep their tile.  The
+ * recovery/CFL family is the stand-alone CFL reduction
+ * (gcs_context_timestep).  best_ms / default_ms (nullable, GCS_TILE_FAMILIES entries, 0 for
  * untuned families) receive the chosen and the default tile's ms per
  * launch sequence.  Needs a context with a background (wind case). */
 int gcs_context_autotune(gcs_context *ctx, const gamera_no_advance_options *options,
@@ -666,7 +669,7 @@ int gcs_mi_tensor_plan_upload(gcs_mi_tensor_plan *plan, const double *fac,
                               const double *potential);
 int gcs_mi_tensor_solve_async(gcs_mi_tensor_plan *plan, void *stream);
 /* Ordering of the SSOR preconditioner (no reference counterpart): 0 the
- * reference's row-by-row sweeps (default; one warp advances a wavefront),
+ * reference's row-by-row sweeps (default; a wavefront, one warp to 64 rows),
  * 1 the same splitting with the unknowns ordered by colour (pole; (row +
  * longitude) parity off the seam column; row parity on it), each colour
  * swept by the whole cluster at once.  Both solve to the configured
@@ -676,11 +679,12 @@ int gcs_mi_tensor_plan_set_ordering(gcs_mi_tensor_plan *plan, int colored);
  * pipeline (available where each CTA of the cluster gets at most 32
  * interior rows and the band's coefficients fit in shared memory; the
  * default on grids of fewer than 17 longitudes), each CTA sweeping its band
- * of rows and passing its edge row to the next CTA; 0 one warp advancing
- * the whole wavefront (the default elsewhere).  Both compute the same
- * preconditioner with the same operations and give identical results.  -1
- * when the plan has no band schedule.  gcs_mi_tensor_plan_schedule returns
- * 1 (band, with the rows per band and the band count), 0 (one warp) or -1. */
+ * of rows and passing its edge row to the next CTA; 0 blocks of 64 rows, one
+ * warp each, on as many CTAs (the default elsewhere, and the faster on every
+ * grid measured).  Both compute the same preconditioner with the same
+ * operations and give identical results.  -1 when the plan has no band
+ * schedule.  gcs_mi_tensor_plan_schedule returns 1 (band, with the rows per
+ * band and the band count), 0 (row blocks) or -1. */
 int gcs_mi_tensor_plan_set_schedule(gcs_mi_tensor_plan *plan, int banded);
 int gcs_mi_tensor_plan_schedule(const gcs_mi_tensor_plan *plan, int *rows_per_band,
                                 int *bands);

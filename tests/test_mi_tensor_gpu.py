@@ -84,18 +84,18 @@ def test_tensor_production_grid():
 
 
 @pytest.mark.parametrize("npl,nt,hemisphere", [
-    (8, 12, 1),     # fewer than 9 longitudes: one diagonal per sweep group, 1 chain
-    (5, 40, -1),    # narrow and taller: 2 chains per lane, southern hemisphere
-    (12, 70, 1),    # 3 chains, groups of 4 diagonals
-    (9, 35, 1),     # the narrowest grid swept 4 diagonals at a time
-    (16, 300, -1),  # more than 256 interior rows: 16 chains per lane
-    (17, 60, 1),    # the narrowest grid swept 8 diagonals at a time
-    (40, 250, -1),  # 8 chains per lane, groups of 8 diagonals
-    (40, 100, 1),   # 4 chains per lane, groups of 8 diagonals
-    (35, 34, -1),   # 1 chain per lane, groups of 8 diagonals
+    (8, 12, 1),     # bands of one row
+    (5, 40, -1),    # bands of three rows, southern hemisphere
+    (12, 70, 1),    # bands of five rows
+    (9, 35, 1),
+    (16, 300, -1),  # the widest grid that starts with bands, of 19 rows
+    (17, 60, 1),    # the narrowest grid that starts with row blocks: one
+    (40, 250, -1),  # four blocks
+    (40, 100, 1),   # two blocks
+    (35, 34, -1),   # half a block
 ])
 def test_tensor_grid_shapes(npl, nt, hemisphere):
-    """Every sweep layout (chains per lane, group size) against the oracle.
+    """Both sweep schedules, as plans start with them, against the oracle.
 
     On these tall, narrow grids two solves that each reach relative residual
     1e-8 differ by up to 9e-8 of max|potential| (the reference's own 1e-8
@@ -231,12 +231,12 @@ def test_colored_ordering_converges_to_the_reference_solution(npl, nt, hemispher
     (8, 12, 1),      # 10 rows: 10 bands of one row
     (17, 60, 1),
     (5, 40, -1),
-    (40, 100, 1),    # one warp with 4 chains per lane
+    (40, 100, 1),
 ])
 def test_band_schedule_is_bitwise(npl, nt, hemisphere):
     """The band-pipelined sweeps (each CTA of the cluster sweeps its band of
     rows; edge rows cross between CTAs through distributed shared memory)
-    against the one-warp wavefront: the same operations on the same
+    against the wavefront of 64-row blocks: the same operations on the same
     operands, so the potential and the stats must agree bit for bit."""
     from gamera_cube_b200 import cases
     L = glib()
@@ -246,7 +246,7 @@ def test_band_schedule_is_bitwise(npl, nt, hemisphere):
     assert L.gcs_mi_tensor_plan_create(C.byref(case.config), C.byref(plan)) == 0
     h, n = C.c_int(), C.c_int()
     try:
-        # the default: bands below 17 longitudes, one warp from 17 on
+        # the default: bands below 17 longitudes, row blocks from 17 on
         assert L.gcs_mi_tensor_plan_schedule(plan, None, None) == (1 if npl < 17 else 0)
         assert L.gcs_mi_tensor_plan_set_schedule(plan, 1) == 0
         assert L.gcs_mi_tensor_plan_schedule(plan, C.byref(h), C.byref(n)) == 1
@@ -270,5 +270,5 @@ def test_band_schedule_is_bitwise(npl, nt, hemisphere):
     assert (sa.iterations, sa.initial_residual, sa.final_residual, sa.converged) == \
         (sb.iterations, sb.initial_residual, sb.final_residual, sb.converged)
     assert np.array_equal(pa, pb)
-    print("band schedule %dx%d: one warp %.2f ms, bands %.2f ms, %d iterations"
+    print("band schedule %dx%d: row blocks %.2f ms, bands %.2f ms, %d iterations"
           % (nt, npl, ta, tb, sb.iterations))

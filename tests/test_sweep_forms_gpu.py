@@ -1,7 +1,8 @@
 """The forms of the step's sweeps and transfers that a plain case does not
 reach: face frames that are not orthonormal (the flux sweep then reads the
-tangents), one launch per family, and state transfers at sizes that leave
-partial blocks."""
+tangents), the short kernels launched per family, light speeds and layer
+counts at the edges, and state transfers at sizes that leave partial blocks
+or fail."""
 import ctypes as C
 
 import numpy as np
@@ -62,8 +63,9 @@ def test_frames(lib, kind, nr, n, factor):
 
 @pytest.mark.parametrize("bulk", [0, 1])
 def test_one_launch_per_family(lib, bulk):
-    """A run of an ensemble (one launch per face and edge family) and the
-    same run stepped alone (all families in a launch) agree bit for bit."""
+    """A run of an ensemble (face velocities and CT launched per family, the
+    seam sync per time level) and the same run stepped alone (all in a launch)
+    agree bit for bit."""
     driver = abi.WindDriver(7.0, -420.0, 9e4, -4.0)
     nr, n = (C.c_size_t * 1)(26), (C.c_size_t * 1)(11)
     config = abi.EnsembleConfig()
