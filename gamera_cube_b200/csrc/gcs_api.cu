@@ -114,6 +114,9 @@ bool make_opts(const gamera_no_advance_options *o, bool have_background,
   O.e_rho_floor = e.density_floor;
   O.e_pdm = e.pdm_coefficient;
   O.e_diff = e.diffusion_coefficient;
+  // beyond 1e75 the correction is below rounding for every Alfven speed up
+  // to 1e67, and c^2 stays far from overflow
+  O.e_c = std::fmin(e.light_speed, 1e75);
   O.e_ic2 = e.use_boris ? 1.0 / (e.light_speed * e.light_speed) : 0.0;
   O.e_cfl = e.cfl;
   O.e_boris = e.use_boris;

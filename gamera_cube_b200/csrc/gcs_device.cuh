@@ -144,7 +144,7 @@ struct Opts {
   double s_igm1, s_ic2;          // 1 / (gamma - 1); 1 / c^2 with Boris, else 0
   float s_igm1_f32;              // 1 / (gamma - 1) of the FP32 gamma, in FP32
   bool s_mhd, hogs, s_boris, s_bg;
-  double e_rho_floor, e_pdm, e_diff, e_ic2, e_cfl;  // e_ic2 as s_ic2
+  double e_rho_floor, e_pdm, e_diff, e_c, e_ic2, e_cfl;  // e_ic2 as s_ic2
   bool e_boris, e_bg;
   double u_gamma, u_rho_floor, u_p_floor, u_c;
   bool u_mhd, u_boris, u_bg;

@@ -301,8 +301,9 @@ __device__ __forceinline__ void edge_thread(const Dims &D, const DevState &S,
   const bool rho_ok = isfinite(rho) && rho > DBL_MIN;
   T emf;
   const bool emf_ok =
-      edge_emf(vt1, vt2, ef0, ef1, jump, (T)rho, B.elen[e][cb], (T)O.e_diff,
-               (T)O.e_ic2, (T)(O.e_cfl * Num<double>::rcp(prm->dt)), &emf) == 0;
+      edge_emf(vt1, vt2, ef0, ef1, jump, (T)rho, B.elen[e][cb], (T)O.e_diff, O.e_boris,
+               sizeof(T) == 8 ? (T)O.e_c : (T)O.e_ic2,
+               (T)(O.e_cfl * Num<double>::rcp(prm->dt)), &emf) == 0;
   if (stopped(first, kPassEmf)) return;
   if (geometry != 0 || !rho_ok || !emf_ok) {
     fail(st, geometry != 0 ? geometry : !rho_ok ? kStageEdgeDensity : kStageEdgeEmf, e, f,
